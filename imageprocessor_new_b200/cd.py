@@ -90,26 +90,7 @@ def _projection_operators(size: int):
     return _PROJECTION_OPS[key]
 
 
-_ZOOM_FACTOR = 4
-_ZOOM_OPS: dict = {}
-
-
-def _zoom_operator(size: int) -> torch.Tensor:
-    """(size * 4, size) operator of the half_area family's enlargement along one axis: column i is
-    scipy.ndimage.zoom (order 3, grid mode, zero outside) of the unit profile at i padded with 32
-    zeros either side, cut back to the profile (subpx/_cpu/invariant_cd.py:424-444). On the device."""
-    key = (int(size), torch.cuda.current_device())
-    if key not in _ZOOM_OPS:
-        from scipy.ndimage import zoom
-
-        cols = []
-        for i in range(size):
-            e = np.zeros(size + 2 * _ZERO_PAD)
-            e[_ZERO_PAD + i] = 1.0
-            z = zoom(e, _ZOOM_FACTOR, order=3, mode="grid-constant", grid_mode=True)
-            cols.append(z[_ZERO_PAD * _ZOOM_FACTOR:(_ZERO_PAD + size) * _ZOOM_FACTOR])
-        _ZOOM_OPS[key] = dev.upload(np.ascontiguousarray(np.stack(cols, axis=1)))
-    return _ZOOM_OPS[key]
+_ZOOM_FACTOR = 4  # the area methods' enlargement (built into spx_half_area_spline_cd and spx_tail_area_spline_cd)
 
 
 def _validate(img, *, methods, background, seeds, threshold, area_min, area_max, pad, n_angles, radial_step,
@@ -641,8 +622,6 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
     half = [m for m in methods if m in HALF_AREA]
     t_half = time.perf_counter()
     if half and nr:
-        zy, zx = _zoom_operator(c.hm), _zoom_operator(c.wm)
-        ws = dev.workspace(_lib.size("spx_half_area_workspace_bytes", c.hm, c.wm, _ZOOM_FACTOR))
         big_px = c.hm * c.wm * _ZOOM_FACTOR * _ZOOM_FACTOR
         n_top = min(max(1, int(round(half_area_peak_pixels * _ZOOM_FACTOR * _ZOOM_FACTOR))), big_px)
         for kind in ("median", "min"):
@@ -654,10 +633,10 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
                 hb_ = _method_buffers(nr, n_angles, m, not metrics_only)
                 bufs[m] = hb_[0]
                 outs[HALF_AREA[m][1]] = hb_[1]
-            _lib.call("spx_half_area_cd", cleaned.data_ptr(), c.voronoi.data_ptr(), c.boxes.data_ptr(),
-                      report_d.data_ptr(), nr, c.hm, c.wm, width, n_angles, zy.data_ptr(), zx.data_ptr(), _ZOOM_FACTOR,
-                      float(half_area_level), int(kind == "median"), n_top, int(bool(outlines) and not metrics_only),
-                      outs.get(False), outs.get(True), ws.data_ptr(), ws.numel(), stream)
+            _lib.call("spx_half_area_spline_cd", cleaned.data_ptr(), c.voronoi.data_ptr(), c.boxes.data_ptr(),
+                      report_d.data_ptr(), nr, c.hm, c.wm, width, n_angles, float(half_area_level),
+                      int(kind == "median"), n_top, int(bool(outlines) and not metrics_only), outs.get(False),
+                      outs.get(True), stream)
             launched(names)
     seconds["half_area"] = time.perf_counter() - t_half
     tails = [m for m in methods if m in TAIL_AREA]
@@ -785,7 +764,7 @@ def _tail_areas(img_d, sign, state, c, report, report_d, pitch, names, *, n_angl
                 outlines, metrics_only, meta):
     """The tail family of the reported holes (subpx/_cpu/invariant_cd.py:1009-1068): windows of
     ceil(window x pitch) px half-width holding each hole's share of the light (spx_wide_cells), then
-    spx_tail_area_cd on them, in chunks of holes; foot_area_ratio takes a second pass with the median
+    spx_tail_area_spline_cd on them, in chunks of holes; foot_area_ratio takes a second pass with the median
     foot ratio of the first. Returns the methods' device buffers."""
     nr = len(report)
     # measure_invariant's pitch: the deblend's, else (fewer than two holes) the stack's larger side.
@@ -797,8 +776,6 @@ def _tail_areas(img_d, sign, state, c, report, report_d, pitch, names, *, n_angl
     params = state.params
     good_amp = params[np.isfinite(params).all(axis=1), 0]
     floor = 1e-3 * float(np.median(good_amp)) if good_amp.size else 1e-12
-    zy = _zoom_operator(side)
-    zx_t = zy.t().contiguous()  # one operator per axis (square windows)
     big_px = side * side * _ZOOM_FACTOR * _ZOOM_FACTOR
     n_top = min(max(1, int(round(peak_pixels * _ZOOM_FACTOR * _ZOOM_FACTOR))), big_px)
     first = [m for m in names if m != "foot_area_ratio"]
@@ -810,7 +787,6 @@ def _tail_areas(img_d, sign, state, c, report, report_d, pitch, names, *, n_angl
     cell_org = c.boxes[report_d.to(torch.int64), :2].contiguous()
     chunk = max(1, min(nr, _TAIL_CHUNK_BYTES // (7 * side * side)))
     ws_wide = dev.workspace(_lib.size("spx_wide_cells_workspace_bytes", n_all, chunk, h, w, pitch_t))
-    ws_tail = dev.workspace(_lib.size("spx_tail_area_workspace_bytes", side, _ZOOM_FACTOR, n_angles))
     win_cells = dev.empty((chunk, side, side), torch.float32)
     inside = dev.empty((chunk, side, side), torch.uint8)
     level_px = dev.empty((chunk, side, side), torch.uint8)
@@ -829,11 +805,9 @@ def _tail_areas(img_d, sign, state, c, report, report_d, pitch, names, *, n_angl
                       ws_wide.numel(), stream)
             outs = [(_method_out_rows(bufs[k][0], s0) if k in kinds else None)
                     for k in ("tail_area", "tail_area_norm", "edge_area", "foot_area", "foot_area_ratio")]
-            _lib.call("spx_tail_area_cd", win_cells.data_ptr(), inside.data_ptr(), level_px.data_ptr(),
+            _lib.call("spx_tail_area_spline_cd", win_cells.data_ptr(), inside.data_ptr(), level_px.data_ptr(),
                       territory.data_ptr(), win_org.data_ptr(), cell_org[s0:].data_ptr(), m, side, n_angles,
-                      zy.data_ptr(), zx_t.data_ptr(), _ZOOM_FACTOR, float(level), n_top, int(outlines),
-                      None if cuts is None else cuts[s0:].data_ptr(), *outs, ws_tail.data_ptr(), ws_tail.numel(),
-                      stream)
+                      float(level), n_top, int(outlines), None if cuts is None else cuts[s0:].data_ptr(), *outs, stream)
 
     run(first)
     meta["tail_window_px"] = int(side)

@@ -15,14 +15,15 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "area.cuh"
 #include "lm.cuh"
+#include "methods.cuh"
 #include "select.cuh"
 
 namespace spx {
 namespace {
 
 constexpr double kFwhmK = 1.1774100225154747;  // sqrt(2 ln 2)
-constexpr double kPi = 3.141592653589793;
 constexpr int kPad = 12;
 
 // ------------------------------------------------------------------------------ 2x2 eigh
@@ -117,55 +118,6 @@ __device__ Eig2 eigh2(double a, double b, double c) {
 }
 
 // ---------------------------------------------------------------------------- shared pieces
-
-struct CellView {
-    const double* roi;  // hm x wm cleaned cell (zero outside its mask)
-    const int* vor;
-    int4 box;
-    int j;              // cell index in the Voronoi labels
-    int W, hm, wm;
-    __device__ __forceinline__ bool mask(int yy, int xx) const {
-        return yy >= 0 && xx >= 0 && yy < box.w && xx < box.z && yy < hm && xx < wm &&
-               vor[(long long)(box.y + yy) * W + (box.x + xx)] == j;
-    }
-};
-
-// Output slots of one method (per cell arrays; null pointers are skipped).
-struct MethodOut {
-    double* centers;     // n x 2 global
-    double* contours;    // n x (n_angles + 1) x 2 global, or null (metrics_only)
-    uint8_t* status;     // n
-    double* metrics;     // n x n_metrics, NaN where not measured
-    double* center_local;  // n x 2 (radial, logquad)
-    double* edge_px;     // n x n_angles (radial)
-    double* eigenvalues; // n x 2 (ellipse methods)
-    double* axes;        // n x 2 x 2 (ellipse methods)
-    int n_metrics;
-    long long col_stride;  // 0: row-major metrics; else metric q of cell i at metrics[i + q * col_stride]
-    __device__ __forceinline__ struct MetricRow row(long long i) const;
-};
-
-// One cell's metrics, row-major or column-major.
-struct MetricRow {
-    double* p;
-    long long step;
-    __device__ __forceinline__ double& operator[](int q) const { return p[q * step]; }
-};
-
-__device__ __forceinline__ MetricRow MethodOut::row(long long i) const {
-    return col_stride ? MetricRow{metrics + i, col_stride} : MetricRow{metrics + i * n_metrics, 1};
-}
-
-// Metric columns (same order as the Python side).
-enum {
-    M_AREA = 0, M_CD_EQ = 1, M_CD_X = 2, M_CD_Y = 3, M_PERIM = 4, M_BACKGROUND = 5, M_PEAK = 6,
-    // ellipse methods
-    M_SIG_MAJ = 7, M_SIG_MIN = 8, M_FWHM_MAJ = 9, M_FWHM_MIN = 10, M_ANGLE = 11, M_RMSE = 12,
-    // area methods
-    M_LOCAL_LEVEL = 7, M_THRESHOLD = 8, M_MEAN_SIGNAL = 9, M_STEEPEST = 10,
-    // radial methods
-    M_COVERAGE = 7
-};
 
 // Half-maximum ellipse: contour vertex k of center + (cos t_k, sin t_k) * (K sigma) @ axes^T.
 __device__ __forceinline__ void ellipse_vertex(double cx, double cy, const Eig2& e, double s0, double s1, double ang,
@@ -1448,64 +1400,6 @@ __global__ void k_rebuild_contours(int kind, const double* centers, const double
 
 // ------------------------------------------------------------------------------ projection
 
-// numpy's sum of n values a[k * stride] along a contiguous axis (pairwise_sum): in order below 8
-// values; up to 128, eight running sums (a[j], a[j + 8], ...) combined as ((r0 + r1) + (r2 + r3)) +
-// ((r4 + r5) + (r6 + r7)), then the values past the last full eight in order; above 128, the two
-// halves (the first a multiple of 8 long) summed that way and added.
-__device__ double np_pairwise_sum(const double* a, int n, int stride) {
-    if (n < 8) {
-        double r = 0.0;
-        for (int i = 0; i < n; ++i) r = __dadd_rn(r, a[i * stride]);
-        return r;
-    }
-    if (n <= 128) {
-        double r[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) r[j] = a[j * stride];
-        int i = 8;
-        for (; i < n - (n % 8); i += 8)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = __dadd_rn(r[j], a[(i + j) * stride]);
-        double res = __dadd_rn(__dadd_rn(__dadd_rn(r[0], r[1]), __dadd_rn(r[2], r[3])),
-                               __dadd_rn(__dadd_rn(r[4], r[5]), __dadd_rn(r[6], r[7])));
-        for (; i < n; ++i) res = __dadd_rn(res, a[i * stride]);
-        return res;
-    }
-    int n2 = n / 2;
-    n2 -= n2 % 8;
-    return __dadd_rn(np_pairwise_sum(a, n2, stride), np_pairwise_sum(a + n2 * stride, n - n2, stride));
-}
-
-// np_pairwise_sum by one warp (every lane calls it; all lanes return the sum): lanes 0-7 run the
-// eight running sums of a block of up to 128 values, every lane combines them in numpy's tree and
-// adds the tail; above 128 values the same halves as numpy's.
-__device__ double warp_np_sum(const double* a, int n) {
-    if (n > 128) {
-        int n2 = n / 2;
-        n2 -= n2 % 8;
-        const double left = warp_np_sum(a, n2);
-        return __dadd_rn(left, warp_np_sum(a + n2, n - n2));
-    }
-    if (n < 8) {
-        double r = 0.0;
-        for (int i = 0; i < n; ++i) r = __dadd_rn(r, a[i]);
-        return r;
-    }
-    const int lane = threadIdx.x & 31, full = n - n % 8;
-    double r = 0.0;
-    if (lane < 8) {
-        r = a[lane];
-        for (int i = 8; i < full; i += 8) r = __dadd_rn(r, a[i + lane]);
-    }
-    double q[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) q[j] = __shfl_sync(0xffffffffu, r, j);
-    double res = __dadd_rn(__dadd_rn(__dadd_rn(q[0], q[1]), __dadd_rn(q[2], q[3])),
-                           __dadd_rn(__dadd_rn(q[4], q[5]), __dadd_rn(q[6], q[7])));
-    for (int i = full; i < n; ++i) res = __dadd_rn(res, a[i]);
-    return res;
-}
-
 constexpr int kProjWarps = 4;
 
 // The "projection" CD of each cell (subpx/_cpu/invariant_cd.py:365-421), one warp per cell: the x
@@ -1708,7 +1602,6 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_projection_cd(
 // ------------------------------------------------------------------------------ half_area family
 
 constexpr int kHalfThreads = 256;
-constexpr int kHalfLeavesMax = 1024;  // pairwise-sum leaves of one enlarged cell (<= 128 values each)
 constexpr int kHalfCtas = 148 * 4;    // persistent CTAs (each with its own scratch)
 
 // The leaves of numpy's pairwise sum of n values (blocks of at most 128, split at half rounded down to
@@ -1732,16 +1625,6 @@ __device__ double np_pairwise_tree(const double* leaf, int n, int* next) {
     n2 -= n2 % 8;
     const double a = np_pairwise_tree(leaf, n2, next);
     return __dadd_rn(a, np_pairwise_tree(leaf, n - n2, next));
-}
-
-// Doubles before the zoom operators in a half-area CTA's shared memory: cell, ring, leaf sums and
-// small arrays (doubles), four bit planes, row / column counts and leaves (ints), the mask bytes.
-__host__ __device__ inline long long half_ops_offset(int hm, int wm, int f, int n_angles) {
-    const long long Hb = (long long)hm * f, Wb = (long long)wm * f, RW = (Wb + 31) / 32, area = (long long)hm * wm;
-    const long long tmpn = Hb + Wb > 3LL * (n_angles + 1) ? Hb + Wb : 3LL * (n_angles + 1);
-    const long long bytes = (2 * area + kHalfLeavesMax + tmpn) * 8 + 4 * Hb * RW * 4 + (Hb + Wb + 2 * kHalfLeavesMax) * 4 +
-                            area;
-    return (bytes + 7) / 8;
 }
 
 struct HalfArgs {
@@ -1780,13 +1663,6 @@ struct HalfCtx {
     int top;
     int* s_int;
     double* s_dbl;
-};
-
-// Where an area output's positions go: centres and contours are the enlargement's local positions
-// plus (ox, oy); center_local is the local position itself, or with a finite lx the global centre
-// minus (lx, ly) (the tail windows report it relative to the hole's own cell).
-struct AreaPlace {
-    double ox, oy, lx, ly;
 };
 
 // One output of the area methods from the cell's enlargement: region above b + cut around the
@@ -1935,7 +1811,6 @@ __device__ void half_output(const HalfArgs& a, const MethodOut& out, int i, doub
     const double cy = __ddiv_rn(h.s_dbl[0], weight), cx = __ddiv_rn(h.s_dbl[1], weight);
     const double mean_signal = __ddiv_rn(h.s_dbl[2], weight);
     const double sx = 1.0 / a.factor, sy = sx;
-    const bool pow2 = (a.factor & (a.factor - 1)) == 0;
     for (int X = tid; X < Wb; X += kHalfThreads) {
         const double d = __dsub_rn((double)X, cx);
         tx[X] = __dmul_rn((double)h.colcnt[X], __dmul_rn(d, d));
@@ -1954,103 +1829,10 @@ __device__ void half_output(const HalfArgs& a, const MethodOut& out, int i, doub
     }
     __syncthreads();
     const double var_x = h.s_dbl[3], var_y = h.s_dbl[2];
-    const double shift = (double)(a.factor - 1) / (2.0 * a.factor);
-    const double cxl = __dsub_rn(__dmul_rn(cx, sx), shift), cyl = __dsub_rn(__dmul_rn(cy, sy), shift);
-    const bool ok = signal && !touch;
-    // Display outline: along each ray from the centroid, the last 1/8 px step still in the region.
-    const int nv = a.n_angles + 1;
-    double* vx = h.tmp;
-    double* vy = h.tmp + nv;
-    if (a.outlines && signal) {
-        const int nr = (int)ceil(hypot((double)a.hm, (double)a.wm) / 0.125);
-        const double ang_step = 2.0 * kPi / a.n_angles;
-        for (int q = tid; q < a.n_angles; q += kHalfThreads) {
-            const double ang = __dmul_rn((double)q, ang_step);
-            const double co = cos(ang), si = sin(ang);
-            int first_out = nr;
-            for (int s = 0; s < nr; ++s) {
-                const double st = __dmul_rn((double)s, 0.125);
-                // (cos x step) / sx, a multiplication by the factor when it is a power of two (exact).
-                const double ox = pow2 ? __dmul_rn(__dmul_rn(co, st), (double)a.factor) : __ddiv_rn(__dmul_rn(co, st), sx);
-                const double oy = pow2 ? __dmul_rn(__dmul_rn(si, st), (double)a.factor) : __ddiv_rn(__dmul_rn(si, st), sy);
-                const double fx = rint(__dadd_rn(cx, ox));
-                const double fy = rint(__dadd_rn(cy, oy));
-                bool hit = fx >= 0.0 && fx < (double)Wb && fy >= 0.0 && fy < (double)Hb;
-                if (hit) {
-                    const int X = (int)fx, Y = (int)fy;
-                    hit = (cur[Y * RW + X / 32] >> (X % 32)) & 1u;
-                }
-                if (!hit) {
-                    first_out = s;
-                    break;
-                }
-            }
-            const double e = __dadd_rn(__dmul_rn((double)max(first_out - 1, 0), 0.125), 0.0625);
-            if (out.edge_px) out.edge_px[(long long)i * a.n_angles + q] = e;
-            vx[q] = __dadd_rn(__dadd_rn(cxl, __dmul_rn(e, co)), at.ox);
-            vy[q] = __dadd_rn(__dadd_rn(cyl, __dmul_rn(e, si)), at.oy);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            vx[a.n_angles] = vx[0];
-            vy[a.n_angles] = vy[0];
-        }
-        __syncthreads();
-        if (out.contours)
-            for (int k = tid; k < nv; k += kHalfThreads) {
-                out.contours[((long long)i * nv + k) * 2] = vx[k];
-                out.contours[((long long)i * nv + k) * 2 + 1] = vy[k];
-            }
-        // Perimeter: the closed polygon's side lengths, summed in numpy's order by one warp.
-        double* side = h.tmp + 2 * nv;
-        for (int q = tid; q < a.n_angles; q += kHalfThreads) {
-            const double dx = __dsub_rn(vx[q + 1], vx[q]), dy = __dsub_rn(vy[q + 1], vy[q]);
-            side[q] = sqrt(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-        }
-        __syncthreads();
-        if (warp == 0) {
-            const double v = warp_np_sum(side, a.n_angles);
-            if (lane == 0) h.s_dbl[3] = v;
-        }
-    } else {
-        if (out.edge_px)
-            for (int q = tid; q < a.n_angles; q += kHalfThreads) out.edge_px[(long long)i * a.n_angles + q] = dnan();
-        if (out.contours)
-            for (int k = tid; k < 2 * nv; k += kHalfThreads) out.contours[(long long)i * 2 * nv + k] = dnan();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const MetricRow m = out.row(i);
-        for (int q = 0; q < out.n_metrics; ++q) m[q] = dnan();
-        m[M_LOCAL_LEVEL] = h.b;
-        out.status[i] = (uint8_t)(!signal ? SPX_ST_NO_SIGNAL : touch ? SPX_ST_REGION_AT_CELL_BORDER : SPX_ST_OK);
-        const double nan = dnan();
-        const double gcx = __dadd_rn(cxl, at.ox), gcy = __dadd_rn(cyl, at.oy);
-        out.centers[2LL * i] = signal ? gcx : nan;
-        out.centers[2LL * i + 1] = signal ? gcy : nan;
-        if (out.center_local) {
-            const bool rel = isfinite(at.lx);
-            out.center_local[2LL * i] = signal ? (rel ? __dsub_rn(gcx, at.lx) : cxl) : nan;
-            out.center_local[2LL * i + 1] = signal ? (rel ? __dsub_rn(gcy, at.ly) : cyl) : nan;
-        }
-        if (signal) {
-            m[M_PEAK] = peak;
-            m[M_THRESHOLD] = __dadd_rn(h.b, cut);
-            m[M_MEAN_SIGNAL] = mean_signal;
-            if (out.n_metrics > M_STEEPEST) m[M_STEEPEST] = steepest;
-        }
-        if (ok) {
-            const double area = __dmul_rn((double)count, __dmul_rn(sx, sy));
-            const double cd_eq = __dmul_rn(2.0, sqrt(__ddiv_rn(area, kPi)));
-            const double ratio = sqrt(sqrt(__ddiv_rn(fmax(var_x, 1e-12), fmax(var_y, 1e-12))));
-            m[M_AREA] = area;
-            m[M_CD_EQ] = cd_eq;
-            m[M_CD_X] = __dmul_rn(cd_eq, ratio);
-            m[M_CD_Y] = __ddiv_rn(cd_eq, ratio);
-            if (a.outlines) m[M_PERIM] = h.s_dbl[3];
-        }
-    }
-    __syncthreads();
+    area_result<kHalfThreads>(AreaShape{a.hm, a.wm, a.n_angles, a.factor, a.outlines}, out, i,
+                              AreaFound{signal, touch != 0, count, cx, cy, var_x, var_y, mean_signal, peak, cut, h.b,
+                                        steepest},
+                              cur, RW, h.tmp, h.s_dbl + 3, at);
 }
 
 // The half_area family (subpx/_cpu/invariant_cd.py:551-799 with 802-875 for the level backgrounds):
@@ -2373,16 +2155,6 @@ struct TailArgs {
     const double* cuts;      // (n) foot_area_ratio's thresholds
     MethodOut med, norm, edge, foot, given;  // status null: not wanted
 };
-
-// Shared memory of a tail CTA: the window (doubles), leaf sums and small arrays, five bit planes,
-// row / column counts, the three masks. The enlargement, its first product (whose space also holds
-// the level pixels' values before it) and the pairwise-sum leaves live in the CTA's global scratch,
-// so that two CTAs fit an SM for windows up to 59 px.
-__host__ __device__ inline long long tail_smem_bytes(int S, int f, int n_angles) {
-    const long long Hb = (long long)S * f, RW = (Hb + 31) / 32, area = (long long)S * S;
-    const long long tmpn = 2 * Hb > 3LL * (n_angles + 1) ? 2 * Hb : 3LL * (n_angles + 1);
-    return (area + 2 * kHalfLeavesMax + tmpn) * 8 + 5 * Hb * RW * 4 + 2 * Hb * 4 + 3 * area;
-}
 
 // Doubles of one tail CTA's global scratch: enlargement (Hb^2), first product (Hb S), leaves.
 __host__ __device__ inline long long tail_scratch_doubles(int S, int f) {
@@ -2718,25 +2490,6 @@ __global__ void k_status_text(const uint8_t* codes, int n, uint32_t* out) {
     }
 }
 
-MethodOut method_out(const spx_method_out* o) {
-    MethodOut m;
-    if (!o) {
-        m = MethodOut{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0};
-        return m;
-    }
-    m.centers = o->centers;
-    m.contours = o->contours;
-    m.status = o->status;
-    m.metrics = o->metrics;
-    m.center_local = o->center_local;
-    m.edge_px = o->edge_px;
-    m.eigenvalues = o->eigenvalues;
-    m.axes = o->axes;
-    m.n_metrics = o->n_metrics;
-    m.col_stride = o->metric_col_stride;
-    return m;
-}
-
 }  // namespace
 }  // namespace spx
 
@@ -2805,13 +2558,6 @@ int spx_projection_cd(const double* cleaned, const int* voronoi, const int* boxe
     return check_launch("k_projection_cd");
 }
 
-// Shared memory of one half-area CTA (see the layout in k_half_area): the cell's arrays, then the
-// two zoom operators and the first product.
-static size_t half_smem(int hm, int wm, int f, int n_angles) {
-    return (half_ops_offset(hm, wm, f, n_angles) + (size_t)hm * f * hm + (size_t)wm * f * wm + (size_t)hm * f * wm) *
-           sizeof(double);
-}
-
 size_t spx_half_area_workspace_bytes(int hm, int wm, int factor) {
     const size_t Hb = (size_t)hm * factor, Wb = (size_t)wm * factor;
     return (size_t)kHalfCtas * Hb * Wb * sizeof(double) + 256;
@@ -2830,10 +2576,10 @@ int spx_half_area_cd(const double* cleaned, const int* voronoi, const int* boxes
     // Up to 32768 sub-pixels: numpy's pairwise-sum leaves (at least 57 values each) then fit kHalfLeavesMax.
     SPX_REQUIRE((long long)hm * factor * wm * factor <= 32768, "cell stack too large for the half-area kernel");
     SPX_REQUIRE(workspace_bytes >= spx_half_area_workspace_bytes(hm, wm, factor), "workspace too small");
-    const size_t smem = half_smem(hm, wm, factor, n_angles);
+    const size_t smem = half_area_bytes(hm, wm, factor, n_angles);
     SPX_REQUIRE(smem <= 200 * 1024, "cell stack too large for the half-area kernel");
-    if (smem > 48 * 1024)
-        SPX_CUDA(cudaFuncSetAttribute(k_half_area, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (Always: the kernel's static arrays count towards the 48 KB that need no attribute.)
+    SPX_CUDA(cudaFuncSetAttribute(k_half_area, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uintptr_t base = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~(uintptr_t)255;
     HalfArgs a{cleaned, voronoi, reinterpret_cast<const int4*>(boxes), which, n, hm, wm, width, n_angles, zoom_y,
                zoom_x, factor, level, median, n_top, outlines, reinterpret_cast<double*>(base), method_out(single),
@@ -2848,9 +2594,9 @@ int spx_half_area_cd(const double* cleaned, const int* voronoi, const int* boxes
 // its shared memory allows.
 static int tail_ctas(int side, int factor, int n_angles) {
     const size_t smem = (size_t)tail_smem_bytes(side, factor, n_angles);
-    if (smem > 48 * 1024)
-        if (cudaFuncSetAttribute(k_tail_area, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return 0;
+    // (Always: the kernel's static arrays count towards the 48 KB that need no attribute.)
+    if (cudaFuncSetAttribute(k_tail_area, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tail_area, kHalfThreads, smem) != cudaSuccess) return 0;
     return 148 * std::min(std::max(per_sm, 1), 4);

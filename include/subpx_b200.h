@@ -475,6 +475,12 @@ int spx_half_area_cd(const double* cleaned, const int* voronoi, const int* boxes
                      int wm, int width, int n_angles, const double* zoom_y, const double* zoom_x, int factor,
                      double level, int median, int n_top, int outlines, const spx_method_out* single,
                      const spx_method_out* averaged, void* workspace, size_t workspace_bytes, void* stream);
+/* spx_half_area_cd at factor 4 with measure_cds' own enlargement built in (the cubic B-spline of the cell
+ * with zeros outside, as scipy.ndimage.zoom evaluates it): the same cells, outputs and statuses, no
+ * operators and no workspace. */
+int spx_half_area_spline_cd(const double* cleaned, const int* voronoi, const int* boxes, const int* which, int n, int hm,
+                            int wm, int width, int n_angles, double level, int median, int n_top, int outlines,
+                            const spx_method_out* single, const spx_method_out* averaged, void* stream);
 /* Windows of the tail family (subpx/_cpu/invariant_cd.py:878-964, _wide_cells; replaces its CPU
  * branch and subpx/_gpu/windows.py wide_cells): for each reported hole rows[i] (of n_all modelled holes
  * with ROI-local Gaussian params (n_all, 6) and cell boxes (n_all, 4) of an hm x wm stack) the
@@ -509,6 +515,12 @@ int spx_tail_area_cd(const float* cells, const uint8_t* inside, const uint8_t* l
                      const double* cuts, const spx_method_out* tail, const spx_method_out* norm,
                      const spx_method_out* edge, const spx_method_out* foot, const spx_method_out* given,
                      void* workspace, size_t workspace_bytes, void* stream);
+/* spx_tail_area_cd at factor 4 with measure_cds' own enlargement built in, as spx_half_area_spline_cd. */
+int spx_tail_area_spline_cd(const float* cells, const uint8_t* inside, const uint8_t* level_pixels,
+                            const uint8_t* territory, const int* window_origins, const int* cell_origins, int n, int side,
+                            int n_angles, double level, int n_top, int outlines, const double* cuts,
+                            const spx_method_out* tail, const spx_method_out* norm, const spx_method_out* edge,
+                            const spx_method_out* foot, const spx_method_out* given, void* stream);
 size_t spx_radial_workspace_bytes(int hm, int wm, int smooth);
 /* Cubic-spline radial profiles; half-height crossings (halfmax) and gradient maxima (gradient).
  * Either output may be null. smooth_weights (device, 2 smooth_radius + 1 symmetric Gaussian

@@ -1,0 +1,144 @@
+"""The area kernels with the cubic-spline enlargement built in (spx_half_area_spline_cd,
+spx_tail_area_spline_cd) against the general kernels (spx_half_area_cd, spx_tail_area_cd) given the
+same enlargement as dense operators (scipy's zoom of the unit profiles), over the forms they take:
+cells and windows narrower and wider than a word of sub-pixels and than a CTA's columns, single rows
+and columns, ragged and empty masks, each level, peak and threshold rule, lists that overflow.
+
+Tolerance: the two enlargements differ by a few ulps of the cell's largest value (both are FP64 sums
+of at most a few hundred terms: under 1e-13 of it), so the regions, decisions against a threshold,
+are the same and metrics agree to 1e-10 relative.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ANGLES = 48
+
+
+def _operator(size):
+    from scipy.ndimage import zoom
+
+    cols = []
+    for i in range(size):
+        e = np.zeros(size + 64)
+        e[32 + i] = 1.0
+        cols.append(zoom(e, 4, order=3, mode="grid-constant", grid_mode=True)[128:128 + 4 * size])
+    return np.ascontiguousarray(np.stack(cols, axis=1))
+
+
+def _outputs(n, columns):
+    import torch
+
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    b = {"centers": dev.empty((n, 2), torch.float64), "contours": dev.empty((n, ANGLES + 1, 2), torch.float64),
+         "status": dev.empty((n,), torch.uint8), "metrics": dev.empty((columns, n), torch.float64),
+         "center_local": dev.empty((n, 2), torch.float64), "edge_px": dev.empty((n, ANGLES), torch.float64)}
+    struct = _lib.MethodOut(b["centers"].data_ptr(), b["contours"].data_ptr(), b["status"].data_ptr(),
+                            b["metrics"].data_ptr(), b["center_local"].data_ptr(), b["edge_px"].data_ptr(), None, None,
+                            columns, n)
+    return b, struct
+
+
+def _same(a, b):
+    np.testing.assert_array_equal(a["status"].cpu().numpy(), b["status"].cpu().numpy())
+    for key in ("metrics", "centers", "center_local", "contours", "edge_px"):
+        np.testing.assert_allclose(a[key].cpu().numpy(), b[key].cpu().numpy(), rtol=1e-10, atol=1e-10, err_msg=key)
+
+
+def _cells(n, hm, wm, rng):
+    """Noisy blobs, the last ones flat, dark, saturated and without a mask; ragged masks."""
+    y, x = np.mgrid[:hm, :wm]
+    cells = np.empty((n, hm, wm))
+    masks = np.empty((n, hm, wm), bool)
+    for i in range(n):
+        cy, cx = (hm - 1) / 2 + rng.uniform(-1, 1), (wm - 1) / 2 + rng.uniform(-1, 1)
+        r = np.hypot((y - cy) / max(1.0, hm / 4), (x - cx) / max(1.0, wm / 4))
+        cells[i] = 3000.0 / (1 + np.exp(6 * (r - 1))) + rng.normal(0, 60, (hm, wm))
+        masks[i] = (np.abs(y - cy) <= 0.47 * hm) & (rng.random((hm, wm)) < (1.0 if i % 2 else 0.97))
+    cells[n - 4] = 500.0
+    cells[n - 3] = -cells[n - 3]
+    cells[n - 2] = np.minimum(cells[n - 2], 1500.0)
+    masks[n - 1] = False
+    return cells, masks
+
+
+@pytest.mark.parametrize("hm, wm", [(1, 1), (3, 5), (8, 8), (9, 33), (18, 18), (24, 24), (31, 32), (33, 30), (36, 36), (2, 60)])
+@pytest.mark.parametrize("median, n_top, outlines", [(1, 64, 1), (0, 7, 0), (0, 1 << 20, 1)])
+def test_half_area_spline_matches_the_dense_operators(hm, wm, median, n_top, outlines):
+    import torch
+
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    rng = np.random.default_rng(100 * hm + wm)
+    n = 9
+    cells, masks = _cells(n, hm, wm, rng)
+    vor = np.where(masks, np.arange(n)[:, None, None], -1).astype(np.int32).reshape(n * hm, wm)
+    boxes = np.column_stack((np.zeros(n), np.arange(n) * hm, np.full(n, wm), np.full(n, hm))).astype(np.int32)
+    roi = dev.upload(np.where(masks, cells, 0.0))
+    vor_d, boxes_d = dev.upload(vor), dev.upload(boxes)
+    zy, zx = dev.upload(_operator(hm)), dev.upload(_operator(wm))
+    n_top = min(n_top, hm * wm * 16)
+    got, want = [], []
+    for dense in (False, True):
+        (s, ss), (m, ms) = _outputs(n, 13), _outputs(n, 13)
+        (want if dense else got).extend((s, m))
+        head = (roi.data_ptr(), vor_d.data_ptr(), boxes_d.data_ptr(), None, n, hm, wm, wm, ANGLES)
+        if dense:
+            ws = dev.workspace(_lib.size("spx_half_area_workspace_bytes", hm, wm, 4))
+            _lib.call("spx_half_area_cd", *head, zy.data_ptr(), zx.data_ptr(), 4, 0.5, median, n_top, outlines, ss, ms,
+                      ws.data_ptr(), ws.numel(), dev.stream_ptr())
+        else:
+            _lib.call("spx_half_area_spline_cd", *head, 0.5, median, n_top, outlines, ss, ms, dev.stream_ptr())
+        torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        _same(a, b)
+    if hm >= 8 and wm >= 8:
+        assert (got[0]["status"].cpu().numpy() != 1).sum() >= 5  # regions were found
+
+
+@pytest.mark.parametrize("side", [1, 3, 8, 21, 32, 33, 59, 64])
+@pytest.mark.parametrize("n_top, outlines", [(64, 1), (3000, 0)])
+def test_tail_area_spline_matches_the_dense_operators(side, n_top, outlines):
+    import torch
+
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    rng = np.random.default_rng(side)
+    n = 8
+    cells, _ = _cells(n, side, side, rng)
+    y, x = np.mgrid[:side, :side]
+    inside = np.ones((n, side, side), np.uint8)
+    inside[0, :, : side // 3] = 0  # windows past the image's left and lower edge
+    inside[1, 2 * side // 3:, :] = 0
+    r = np.hypot(y - (side - 1) / 2, x - (side - 1) / 2)
+    level = np.broadcast_to((r > 0.42 * side).astype(np.uint8), inside.shape).copy()
+    zone = np.broadcast_to((r < 0.45 * side).astype(np.uint8), inside.shape).copy()
+    level[2] = 0  # no level pixels
+    up = [dev.upload(np.ascontiguousarray(a)) for a in (cells.astype(np.float32), inside, level, zone)]
+    org = dev.upload(rng.integers(-3, 900, (n, 2)).astype(np.int32))
+    cell_org = dev.upload(rng.integers(0, 900, (n, 2)).astype(np.int32))
+    cuts = dev.upload(rng.uniform(100.0, 900.0, n))
+    op = _operator(side)
+    zy, zx_t = dev.upload(op), dev.upload(np.ascontiguousarray(op.T))
+    n_top = min(n_top, side * side * 16)
+    got, want = [], []
+    for dense in (False, True):
+        outs = [_outputs(n, 13) for _ in range(5)]
+        (want if dense else got).extend(b for b, _ in outs)
+        head = [a.data_ptr() for a in up] + [org.data_ptr(), cell_org.data_ptr(), n, side, ANGLES]
+        tail = [0.2, n_top, outlines, cuts.data_ptr()] + [s for _, s in outs]
+        if dense:
+            ws = dev.workspace(_lib.size("spx_tail_area_workspace_bytes", side, 4, ANGLES))
+            _lib.call("spx_tail_area_cd", *head, zy.data_ptr(), zx_t.data_ptr(), 4, *tail, ws.data_ptr(), ws.numel(),
+                      dev.stream_ptr())
+        else:
+            _lib.call("spx_tail_area_spline_cd", *head, *tail, dev.stream_ptr())
+        torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        _same(a, b)
