@@ -52,6 +52,15 @@ class GemmEpilogue(ctypes.Structure):
                 ("out_bf16", c_void_p), ("ld_bf16", c_int), ("out_bf16_t", c_void_p), ("ld_t", c_int)]
 
 
+class MlpTrain(ctypes.Structure):
+    """spx_mlp_train: parameters in the order w1, b1, w2, b2, w3, b3."""
+
+    _fields_ = [("x", c_void_p), ("x_t", c_void_p), ("target", c_void_p), ("weights", c_void_p),
+                ("param", c_void_p * 6), ("grad", c_void_p * 6), ("m", c_void_p * 6), ("v", c_void_p * 6),
+                ("w1", c_void_p), ("w2", c_void_p), ("w2_t", c_void_p), ("w3", c_void_p), ("w3_t", c_void_p),
+                ("loss", c_void_p), ("error_flag", c_void_p)]
+
+
 class FitOptions(ctypes.Structure):
     """spx_fit_options: LM arithmetic (FIT_F64 / FIT_F32), the plain fits' relative cost tolerance and
     the rows per image of a stack (0: one image)."""
@@ -82,6 +91,9 @@ SIGNATURES = {
     "spx_rowsum_bf16": (_I, [_P, _I, _I, _P, _P]),
     "spx_adamw": (_I, [_P, _P, _P, _P, _I, _I, _I, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                        ctypes.c_float, _P, _I, _P, _I, _P]),
+    "spx_mlp_train_workspace_bytes": (_S, [_I]),
+    "spx_mlp_train_step": (_I, [POINTER(MlpTrain), _I, _I, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                                ctypes.c_float, ctypes.c_float, _P, _S, _P]),
     "spx_transpose_bf16": (_I, [_P, _I, _I, _P, _P]),
     "spx_mlp_outputs_to_params": (_I, [_P, _P, _P, _P, _P, _I, _P, _P, _P]),
     "spx_extract_patches": (_I, [_P, _I, _D, _I, _I, _P, _I, _P, _P, _P]),

@@ -118,14 +118,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// 16-byte asynchronous global -> shared copy (zero-filled past src_bytes).
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
-                 :
-                 : "r"(smem_u32(dst_smem)), "l"(src), "r"(src_bytes)
-                 : "memory");
+// Makes freshly initialised mbarriers visible to the async proxy (TMA, tcgen05.commit).
+__device__ __forceinline__ void fence_mbar_init() {
+    asm volatile("fence.mbarrier_init.release.cluster;\n" : : : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" : : : "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" : : : "memory"); }
+
+// Arrives on the mbarrier and adds the bytes that its phase waits for.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" : : "r"(smem_u32(mbar)), "r"(bytes) : "memory");
+}
+
+// TMA load of the box at (x, y) (x the contiguous coordinate) of a 2-D tensor map; its bytes, those past
+// the tensor's edges (zeros) included, complete on the mbarrier. The box starts on 16 bytes: x is a
+// multiple of the K-block.
+__device__ __forceinline__ void tma_load_2d(void* dst_smem, const void* map, int x, int y, uint64_t* mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+        :
+        : "r"(smem_u32(dst_smem)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(mbar))
+        : "memory");
+}
 
 }  // namespace spx

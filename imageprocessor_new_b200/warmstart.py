@@ -127,51 +127,27 @@ class WarmStartNet:
 
     # ---------------------------------------------------------------------------- training
     def train_step(self, x: torch.Tensor, xt: torch.Tensor, t: torch.Tensor, weights: torch.Tensor, *, lr: float,
-                   weight_decay: float = 1e-4, loss_acc: torch.Tensor | None = None) -> torch.Tensor:
+                   weight_decay: float = 1e-4, loss_acc: torch.Tensor | None = None, beta1: float = 0.9,
+                   beta2: float = 0.999, eps: float = 1e-8) -> torch.Tensor:
         """One AdamW step on the batch (x: B x 1024 bf16, xt: its transpose, t: B x 7 standardised
         targets f32; B a multiple of 8). Returns the device loss accumulator (f64)."""
         b = x.shape[0]
-        bf = torch.bfloat16
-        y, (h1, h1t, h2, h2t) = self.forward(x, keep=True)
         if loss_acc is None:
             loss_acc = torch.zeros(1, dtype=torch.float64, device="cuda")
-        dy = dev.empty((b, OUT_PAD), bf)
-        dyt = dev.empty((OUT_PAD, b), bf)
-        _lib.call("spx_mlp_loss_grad", y.data_ptr(), t.data_ptr(), weights.data_ptr(), b, OUT, OUT_PAD, dy.data_ptr(),
-                  dyt.data_ptr(), loss_acc.data_ptr(), dev.stream_ptr())
-        p = self.p
-        # dW3 = dY^T H2, db3 = row sums of dY^T.
-        _gemm(dyt, h2t, OUT, HID, b, out_f32=p["w3"].g, ld_f32=HID, err=self.err)
-        _lib.call("spx_rowsum_bf16", dyt.data_ptr(), OUT, b, p["b3"].g.data_ptr(), dev.stream_ptr())
-        # dH2 = (dY W3) * (H2 > 0), kept transposed for dW2 and row-major for dH1.
-        dh2 = dev.empty((b, HID), bf)
-        dh2t = dev.empty((HID, b), bf)
-        _gemm(dy, self.w3t, b, HID, OUT_PAD, mask=h2, ld_mask=HID, out_bf16=dh2, ld_bf16=HID, out_t=dh2t, ld_t=b,
-              err=self.err)
-        _gemm(dh2t, h1t, HID, HID, b, out_f32=p["w2"].g, ld_f32=HID, err=self.err)
-        _lib.call("spx_rowsum_bf16", dh2t.data_ptr(), HID, b, p["b2"].g.data_ptr(), dev.stream_ptr())
-        # dH1 = (dH2 W2) * (H1 > 0), transposed only.
-        dh1t = dev.empty((HID, b), bf)
-        _gemm(dh2, self.w2t, b, HID, HID, mask=h1, ld_mask=HID, out_t=dh1t, ld_t=b, err=self.err)
-        _gemm(dh1t, xt, HID, IN, b, out_f32=p["w1"].g, ld_f32=IN, err=self.err)
-        _lib.call("spx_rowsum_bf16", dh1t.data_ptr(), HID, b, p["b1"].g.data_ptr(), dev.stream_ptr())
-        self.step += 1
-        self._adamw(lr, weight_decay)
-        return loss_acc
+        params = [self.p[name] for name in ("w1", "b1", "w2", "b2", "w3", "b3")]
 
-    def _adamw(self, lr, weight_decay, beta1=0.9, beta2=0.999, eps=1e-8):
-        s = dev.stream_ptr()
-        p = self.p
-        for name, out, out_rows, out_t, ld_t in (("w1", self.w1, HID, None, 0), ("w2", self.w2, HID, self.w2t, HID),
-                                                 ("w3", self.w3, OUT_PAD, self.w3t, OUT_PAD), ("b1", None, 0, None, 0),
-                                                 ("b2", None, 0, None, 0), ("b3", None, 0, None, 0)):
-            q = p[name]
-            rows, cols = (q.w.shape[0], q.w.shape[1]) if q.w.dim() == 2 else (1, q.w.shape[0])
-            wd = weight_decay if name.startswith("w") else 0.0
-            _lib.call("spx_adamw", q.w.data_ptr(), q.g.data_ptr(), q.m.data_ptr(), q.v.data_ptr(), rows, cols,
-                      self.step, ctypes.c_float(lr), ctypes.c_float(beta1), ctypes.c_float(beta2),
-                      ctypes.c_float(eps), ctypes.c_float(wd), None if out is None else out.data_ptr(),
-                      out_rows, None if out_t is None else out_t.data_ptr(), ld_t, s)
+        def pointers(field):
+            return (ctypes.c_void_p * 6)(*(getattr(q, field).data_ptr() for q in params))
+
+        state = _lib.MlpTrain(x.data_ptr(), xt.data_ptr(), t.data_ptr(), weights.data_ptr(), pointers("w"),
+                              pointers("g"), pointers("m"), pointers("v"), self.w1.data_ptr(), self.w2.data_ptr(),
+                              self.w2t.data_ptr(), self.w3.data_ptr(), self.w3t.data_ptr(), loss_acc.data_ptr(),
+                              self.err.data_ptr())
+        ws = dev.workspace(_lib.size("spx_mlp_train_workspace_bytes", b))
+        _lib.call("spx_mlp_train_step", state, b, self.step + 1, lr, beta1, beta2, eps, weight_decay, ws.data_ptr(),
+                  ws.numel(), dev.stream_ptr())
+        self.step += 1
+        return loss_acc
 
     def check_errors(self):
         if int(self.err.item()):

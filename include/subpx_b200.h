@@ -594,6 +594,23 @@ int spx_rowsum_bf16(const void* src, int rows, int cols, float* out, void* strea
 int spx_adamw(float* param, const float* grad, float* m, float* v, int rows, int cols, int step, float lr, float beta1,
               float beta2, float eps, float weight_decay, void* out_bf16, int out_rows, void* out_bf16_t, int ld_t,
               void* stream);
+/* One training step of the warm-start network (1024 -> 256 -> 256 -> 7, ReLU) on a batch (a multiple of
+ * 8): forward, weighted-MSE gradient (as spx_mlp_loss_grad; loss is added to), weight and bias
+ * gradients, AdamW (step counts from 1; weight_decay on the weights only). Parameters in the order w1,
+ * b1, w2, b2, w3, b3, f32, with their gradients (written) and moments (updated); x batch x 1024 and its
+ * transpose, bf16; the bf16 working copies w1, w2 and its transpose, w3 padded to 16 rows and its
+ * transpose are rewritten from the new parameters. Workspace: spx_mlp_train_workspace_bytes. */
+typedef struct {
+    const void *x, *x_t;
+    const float *target, *weights;
+    float *param[6], *grad[6], *m[6], *v[6];
+    void *w1, *w2, *w2_t, *w3, *w3_t;
+    double* loss;
+    int* error_flag;
+} spx_mlp_train;
+size_t spx_mlp_train_workspace_bytes(int batch);
+int spx_mlp_train_step(const spx_mlp_train* t, int batch, int step, float lr, float beta1, float beta2, float eps,
+                       float weight_decay, void* workspace, size_t workspace_bytes, void* stream);
 /* dst (cols x rows) = src (rows x cols)^T, bf16. */
 int spx_transpose_bf16(const void* src, int rows, int cols, void* dst, void* stream);
 /* Standardised MLP outputs y (n x 7 f32) -> ROI-local LM starting params (n x 6): t = y * std +
