@@ -20,7 +20,7 @@ int check_launch(const char* what);
 struct Tuning {
     int fit_warps = 4;          // warps (cells in flight) per block of the LM fit kernels: 2, 4 or 8
     int fit_blocks_per_sm = 8;  // persistent fit blocks per SM: 2..32
-    int render_tile = 64;       // model render tile edge: 16, 32 or 64 pixels
+    int render_tile = 32;       // model render tile edge: 16, 32 or 64 pixels
     int radial_rays = 2;        // radial profiles, one ray per thread: 0 cached spline window, 2 window read per sample
 };
 Tuning& tuning();

@@ -445,7 +445,8 @@ __global__ void __launch_bounds__(kFitWarpsMax * 32, 2) k_fit_initial(FitArgs a,
 // One deblending iteration for every cell: clean (image - background - (model - own)), LM from the
 // current params, relaxation p + relax * (fitted - p) (non-finite components step 0), status of
 // the relaxed params, and max |step[1:]| (NaN unless the cell is "ok" with a finite fit).
-template <typename T>
+// Px: the pixel type (a dtype branch per load cost 3 % of the kernel).
+template <typename T, typename Px>
 __global__ void __launch_bounds__(kFitWarpsMax * 32, 2) k_fit_iteration(FitArgs a, spx_bgmap bg, const double* model, int radius_cap,
                                 const double* params, double relaxation, double* params_out,
                                 uint8_t* status_out, double* maxstep, int* iters) {
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(kFitWarpsMax * 32, 2) k_fit_iteration(FitArgs 
                 const double aa = e1 * dx + p0[4] * dy, bb = e3 * dy;
                 own = p0[0] * exp(-0.5 * (aa * aa + bb * bb));
             }
-            const double raw = a.img.at(y, x);
+            const double raw = px_at<Px>(a.img, y, x);
             return (raw - bg_at(bg, y, x)) - (model[(long long)y * a.img.W + x] - own);
         });
         double amax = 0.0;
@@ -533,19 +534,26 @@ __global__ void k_render_prep(const double* params, const int4* boxes, int n, in
     if ((threadIdx.x & 31) == 0) atomicMax(rmax, local);
 }
 
-// Render tiles: Tile x Tile pixels per 256-thread block (16: one pixel per thread, 32: four rows
-// per thread, 64: sixteen rows per thread, fewer tiles to gather candidates for), chosen by
-// tuning().render_tile.
+// Render tiles: kRenderTile x kRenderTile pixels per block (16, 32 or 64 px; larger tiles gather their
+// candidates less often).
 constexpr int kRenderCap = 2048;
+constexpr int kRenderThreads = 128;
 
 // model(y, x) = sum over cells (increasing index) whose truncated square covers the pixel, each
 // term A exp(-(a^2 + b^2) / 2) for |x - X0| <= r and |y - Y0| <= r (render_models).
+//
+// Bound: FP64 (one exp per pixel and covering Gaussian, about 2.4 on a 24 px lattice). A warp owns a
+// column of 8 x 4 px patches, so a 37 px square that cuts a patch leaves few of its lanes idle (78 % busy;
+// 32 x 1 px rows: 52 %), and skips candidates that miss its columns with one test. Measured on the 8192 page
+// (116k Gaussians): 64 px tiles, 256 threads, rows of 32: 0.97 ms; patches 0.93 ms; 32 px tiles 0.80 ms, with
+// 128 threads 0.73 ms.
 template <int kRenderTile>
-__global__ void __launch_bounds__(256) k_render(int H, int W, BinGrid g, const double* params,
+__global__ void __launch_bounds__(kRenderThreads) k_render(int H, int W, BinGrid g, const double* params,
                                                const double* centres, const int* radius,
                                                const int* rmax_dev, double* model, int* overflow) {
     __shared__ int cand[kRenderCap];
     __shared__ int s_n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx0 = blockIdx.x * kRenderTile, ty0 = blockIdx.y * kRenderTile;
     const int tx1 = min(tx0 + kRenderTile, W) - 1, ty1 = min(ty0 + kRenderTile, H) - 1;
     if (threadIdx.x == 0) s_n = 0;
@@ -555,9 +563,10 @@ __global__ void __launch_bounds__(256) k_render(int H, int W, BinGrid g, const d
     const int gx1 = bin_index((double)(tx1 + rmax + 1), g.cell, g.gw);
     const int gy0 = bin_index((double)(ty0 - rmax - 1), g.cell, g.gh);
     const int gy1 = bin_index((double)(ty1 + rmax + 1), g.cell, g.gh);
-    for (int gy = gy0; gy <= gy1; ++gy) {
+    // One warp per bin row, so that the rows' chains of loads (offsets, points, radii) run side by side.
+    for (int gy = gy0 + warp; gy <= gy1; gy += kRenderThreads / 32) {
         const int j0 = g.start[gy * g.gw + gx0], j1 = g.start[gy * g.gw + gx1 + 1];
-        for (int k = j0 + threadIdx.x; k < j1; k += blockDim.x) {
+        for (int k = j0 + lane; k < j1; k += 32) {
             const int id = g.id[k];
             const double2 c = g.xy[k];
             const double r = (double)radius[id];
@@ -584,18 +593,21 @@ __global__ void __launch_bounds__(256) k_render(int H, int W, BinGrid g, const d
     }
     __syncthreads();
     // Each candidate's centre, amplitude, precision factors and the integer bounds of its truncated
-    // square are staged once per tile (chunks of 256), so a pixel tests a candidate with integer
+    // square are staged once per tile (a block's threads at a time), so a pixel tests a candidate with integer
     // compares and a term costs one exp. |x - cx| <= r <=> ceil(cx - r) <= x <= floor(cx + r) for
     // integer x and r: x - cx and cx -+ r are exact in FP64 for coordinates below 2^16.
-    __shared__ double s_cx[256], s_cy[256], s_a[256], s_e1[256], s_u2[256], s_e3[256];
-    __shared__ int4 s_box[256];  // x lo, x hi, y lo, y hi
-    constexpr int kRows = kRenderTile * kRenderTile / 256;
-    const int x = tx0 + (threadIdx.x % kRenderTile), yb = ty0 + (threadIdx.x / kRenderTile);
+    __shared__ double s_cx[kRenderThreads], s_cy[kRenderThreads], s_a[kRenderThreads];
+    __shared__ double s_e1[kRenderThreads], s_u2[kRenderThreads], s_e3[kRenderThreads];
+    __shared__ int4 s_box[kRenderThreads];  // x lo, x hi, y lo, y hi
+    constexpr int kCols = kRenderTile / 8;                 // patch columns
+    constexpr int kRows = (kRenderTile / 4) * kCols / (kRenderThreads / 32);   // patches of a warp, one below the other
+    const int px0 = tx0 + 8 * (warp % kCols), py0 = ty0 + 4 * kRows * (warp / kCols);
+    const int x = px0 + (lane & 7), yb = py0 + (lane >> 3);
     double acc[kRows];
 #pragma unroll
     for (int q = 0; q < kRows; ++q) acc[q] = 0.0;
-    for (int c0 = 0; c0 < m; c0 += 256) {
-        const int cn = min(256, m - c0);
+    for (int c0 = 0; c0 < m; c0 += kRenderThreads) {
+        const int cn = min(kRenderThreads, m - c0);
         if ((int)threadIdx.x < cn) {
             const int id = sorted[c0 + threadIdx.x];
             const double* p = params + 6LL * id;
@@ -612,12 +624,13 @@ __global__ void __launch_bounds__(256) k_render(int H, int W, BinGrid g, const d
         __syncthreads();
         for (int k = 0; k < cn; ++k) {
             const int4 bx = s_box[k];
-            if (x < bx.x || x > bx.y) continue;
+            if (bx.x > px0 + 7 || bx.y < px0 || bx.z > py0 + 4 * kRows - 1 || bx.w < py0) continue;
+            const bool in_x = x >= bx.x && x <= bx.y;
             const double dx = (double)x - s_cx[k];
 #pragma unroll
             for (int q = 0; q < kRows; ++q) {
-                const int yq = yb + q * (256 / kRenderTile);
-                if (yq < bx.z || yq > bx.w) continue;
+                const int yq = yb + 4 * q;
+                if (!in_x || yq < bx.z || yq > bx.w) continue;
                 const double dy = (double)yq - s_cy[k];
                 const double aa = s_e1[k] * dx + s_u2[k] * dy, bb = s_e3[k] * dy;
                 const double val = s_a[k] * exp(-0.5 * (aa * aa + bb * bb));
@@ -629,7 +642,7 @@ __global__ void __launch_bounds__(256) k_render(int H, int W, BinGrid g, const d
     if (x < W)
 #pragma unroll
         for (int q = 0; q < kRows; ++q) {
-            const int y = yb + q * (256 / kRenderTile);
+            const int y = yb + 4 * q;
             if (y < H) model[(long long)y * W + x] = acc[q];
         }
 }
@@ -1216,17 +1229,33 @@ int launch_fit_initial(const FitArgs& a0, FitLayout L, cudaStream_t s, const dou
     }
 }
 
+template <typename T, typename Px>
+int launch_fit_iteration_px(const FitArgs& a0, FitLayout L, cudaStream_t s, const spx_bgmap& bg, const double* model,
+                            int radius_cap, const double* params, double relaxation, double* params_out,
+                            uint8_t* status_out, double* maxstep, int* iterations) {
+    return launch_fit(a0, L, s, [&](const FitArgs& fa, size_t smem, int warps, int blocks) -> int {
+        if (smem + kLmSlotBytes > 48 * 1024)
+            SPX_CUDA(cudaFuncSetAttribute(k_fit_iteration<T, Px>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_fit_iteration<T, Px><<<blocks, warps * 32, smem, s>>>(fa, bg, model, radius_cap, params, relaxation,
+                                                                 params_out, status_out, maxstep, iterations);
+        return check_launch("k_fit_iteration");
+    });
+}
+
 template <typename T>
 int launch_fit_iteration(const FitArgs& a0, FitLayout L, cudaStream_t s, const spx_bgmap& bg, const double* model,
                          int radius_cap, const double* params, double relaxation, double* params_out,
                          uint8_t* status_out, double* maxstep, int* iterations) {
-    return launch_fit(a0, L, s, [&](const FitArgs& fa, size_t smem, int warps, int blocks) -> int {
-        if (smem + kLmSlotBytes > 48 * 1024)
-            SPX_CUDA(cudaFuncSetAttribute(k_fit_iteration<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_fit_iteration<T><<<blocks, warps * 32, smem, s>>>(fa, bg, model, radius_cap, params, relaxation,
-                                                             params_out, status_out, maxstep, iterations);
-        return check_launch("k_fit_iteration");
-    });
+    auto go = [&](auto px) {
+        return launch_fit_iteration_px<T, decltype(px)>(a0, L, s, bg, model, radius_cap, params, relaxation, params_out,
+                                                        status_out, maxstep, iterations);
+    };
+    switch (a0.img.dtype) {
+        case SPX_U8: return go(uint8_t{});
+        case SPX_U16: return go(uint16_t{});
+        case SPX_F32: return go(float{});
+        default: return go(double{});
+    }
 }
 
 }  // namespace
@@ -1323,16 +1352,20 @@ int spx_render_model(const double* params, const int* boxes, int n, int height, 
         if (int e = check_launch("k_render_prep")) return e;
     }
     if (int e = bin_build(L.bins, L.centres, 2, nullptr, L.valid, n, s)) return e;
-    const int tile = tuning().render_tile;
+    // The tuned tile where it gives the chip a few blocks per SM, smaller ones on small pages (a 480 x 641 px
+    // page of dense spots has 88 tiles of 64 px and 315 of 32 px: 112 and 34 us, 16 px tiles 20 us).
+    int tile = tuning().render_tile;
+    auto tiles = [&](int t) { return (long long)((width + t - 1) / t) * ((height + t - 1) / t); };
+    while (tile > 16 && tiles(tile) < 4 * 148) tile /= 2;
     const dim3 grid((width + tile - 1) / tile, (height + tile - 1) / tile);
     if (tile == 16)
-        k_render<16><<<grid, 256, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
+        k_render<16><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
                                           L.overflow);
     else if (tile == 64)
-        k_render<64><<<grid, 256, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
+        k_render<64><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
                                           L.overflow);
     else
-        k_render<32><<<grid, 256, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
+        k_render<32><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
                                           L.overflow);
     return check_launch("k_render");
 }

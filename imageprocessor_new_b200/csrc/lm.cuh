@@ -233,17 +233,41 @@ template <typename T>
 __device__ inline int warp_lm_fit(double* p, const T* v, const int* xy, int n, double cap, double amp_cap,
                                   int max_iter, int lane, double* slots, double cost_tol = 1e-12,
                                   double* final_cost = nullptr) {
-    int kept = 0;
-    double cost = warp_normal_pass(p, v, xy, n, lane, slots);
-    if (final_cost) *final_cost = cost;
-    if (!isfinite(cost)) return 0;
-    double lam = 1e-3;
+    int kept = 0, it = 0;
+    double cost = 0.0, lam = 1e-3;
     const double lo = -log(cap), hi = -log(kSigmaMin);
-    int it = 0;
-    for (; it < max_iter; ++it) {
+    double trial[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) trial[i] = p[i];
+    // One copy of the pass and of the solve: the first round evaluates the start, the later ones trials.
+    // (Two copies of them in each fit kernel took instruction-cache misses: initial fits of 116k cells 6.11 ->
+    // 5.66 ms, same bits.)
+    bool first = true, small = false;
+    while (true) {
+        // The trial's sums go to the other slot; a rejected trial leaves the kept slot as it was.
+        const double new_cost = warp_normal_pass(trial, v, xy, n, lane, slots + 27 * (first ? 0 : kept ^ 1));
+        if (first) {
+            first = false;
+            cost = new_cost;
+            if (!isfinite(cost)) break;
+        } else {
+            const bool better = isfinite(new_cost) && new_cost <= cost;
+            const bool done = (better && (cost - new_cost <= cost_tol * fmax(cost, 1e-300))) || small;
+            if (better) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) p[i] = trial[i];
+                lam /= 3.0;
+                cost = new_cost;
+                kept ^= 1;
+            } else {
+                lam *= 4.0;
+            }
+            ++it;
+            if (done || lam > 1e12) break;
+        }
+        if (it >= max_iter) break;
         double step[6];
         damped_solve(slots + 27 * kept, slots + 27 * kept + 21, lam, step);
-        double trial[6];
 #pragma unroll
         for (int i = 0; i < 6; ++i) trial[i] = p[i] + step[i];
         // np.clip semantics: NaN passes through.
@@ -254,23 +278,9 @@ __device__ inline int warp_lm_fit(double* p, const T* v, const int* xy, int n, d
 #pragma unroll
         for (int i = 0; i < 6; ++i) smax = fmax(smax, fabs(step[i]));
         // fmax ignores NaN; a NaN step is not "small" (np.abs(nan) < 1e-7 is False).
-        bool small = smax < 1e-7;
+        small = smax < 1e-7;
 #pragma unroll
         for (int i = 0; i < 6; ++i) small = small && !isnan(step[i]);
-        // The trial's sums go to the other slot; a rejected trial leaves the kept slot as it was.
-        const double new_cost = warp_normal_pass(trial, v, xy, n, lane, slots + 27 * (kept ^ 1));
-        const bool better = isfinite(new_cost) && new_cost <= cost;
-        const bool done = (better && (cost - new_cost <= cost_tol * fmax(cost, 1e-300))) || small;
-        if (better) {
-#pragma unroll
-            for (int i = 0; i < 6; ++i) p[i] = trial[i];
-            lam /= 3.0;
-            cost = new_cost;
-            kept ^= 1;
-        } else {
-            lam *= 4.0;
-        }
-        if (done || lam > 1e12) { ++it; break; }
     }
     __syncwarp();
     if (final_cost) *final_cost = cost;
