@@ -72,6 +72,54 @@ __global__ void k_scan_apply(const int* in, long long n, const int* tile_offsets
         }
 }
 
+// The whole scan by one block, 4096 items a round with the next round's loads in flight.
+__global__ void __launch_bounds__(kScanThreads) k_scan_one_block(const int* in, int n, int* out, int* total) {
+    __shared__ int warp_sums[2][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int next[kScanItems], run = 0;
+    auto load = [&](int base) {
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            const int k = base + (int)threadIdx.x * kScanItems + i;
+            next[i] = k < n ? in[k] : 0;
+        }
+    };
+    load(0);
+    for (int base = 0, phase = 0; base < n; base += kScanTile, phase ^= 1) {
+        int v[kScanItems], acc = 0;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = next[i];
+            acc += v[i];
+        }
+        load(base + kScanTile);  // (in place: items past this round are not written yet)
+        int incl = acc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) warp_sums[phase][warp] = incl;
+        __syncthreads();
+        int w = warp_sums[phase][lane], before = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before += u;
+        }
+        const int tile = __shfl_sync(0xffffffffu, before, 31);
+        int off = run + __shfl_sync(0xffffffffu, before - w, warp) + incl - acc;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            const int k = base + (int)threadIdx.x * kScanItems + i;
+            if (k < n) out[k] = off;
+            off += v[i];
+        }
+        run += tile;
+    }
+    if (threadIdx.x == 0 && total) *total = run;
+}
+
 int exclusive_scan(const int* in, long long n, int* out, int* total, int* scratch, cudaStream_t s) {
     const int tiles = scan_tiles(n);
     if (n <= 0) {
@@ -79,6 +127,10 @@ int exclusive_scan(const int* in, long long n, int* out, int* total, int* scratc
         return SPX_OK;
     }
     SPX_REQUIRE(tiles <= kScanThreads * 64, "scan too large");
+    if (n <= kScanOneBlock) {
+        k_scan_one_block<<<1, kScanThreads, 0, s>>>(in, (int)n, out, total);
+        return check_launch("k_scan_one_block");
+    }
     k_scan_tile_sums<<<tiles, kScanThreads, 0, s>>>(in, n, scratch);
     if (int e = check_launch("k_scan_tile_sums")) return e;
     k_scan_tile_sums_exclusive<<<1, kScanThreads, 0, s>>>(scratch, tiles, total);

@@ -1,5 +1,7 @@
-// Exclusive prefix sum of int32 counts in three launches (block sums, one-block scan of the block
-// sums, per-block scan plus offset). Used for order-preserving compaction and counting sorts.
+// Exclusive prefix sum of int32 counts, for order-preserving compaction and counting sorts. Up to
+// kScanOneBlock items in one launch of one block (latency-bound: the three launches take 9 us and their
+// gaps however few the items, the block 2.1 us at 1,000 items and 5.5 us at 12,000); more in three
+// (block sums, one-block scan of the block sums, per-block scan plus offset).
 #pragma once
 
 #include "common.cuh"
@@ -9,6 +11,7 @@ namespace spx {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanOneBlock = 4 * kScanTile;
 
 __global__ void k_scan_tile_sums(const int* in, long long n, int* tile_sums);
 __global__ void k_scan_tile_sums_exclusive(int* tile_sums, int tiles, int* total);

@@ -42,9 +42,82 @@ __global__ void k_bin_fill(const double* pts, int stride, const int* origin, con
     }
 }
 
+// The counting sort of a small grid by one block, its counters in shared memory.
+constexpr int kBinBlock = 1024;
+constexpr int kBinsOneBlock = 8 * 1024;     // bins (32 KB of counters)
+constexpr int kPointsOneBlock = 16 * 1024;  // points
+
+__global__ void __launch_bounds__(kBinBlock) k_bin_build_small(const double* pts, int stride, const int* origin,
+                                                               const uint8_t* valid, int n, int gw, int gh, double cell,
+                                                               int* start, double2* xy, int* id) {
+    extern __shared__ int count[];  // bins + 1
+    __shared__ int warp_sums[32];
+    const int bins = gw * gh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int b = threadIdx.x; b <= bins; b += kBinBlock) count[b] = 0;
+    __syncthreads();
+    auto each = [&](auto&& fn) {  // four points' loads in flight per thread
+        for (int i0 = threadIdx.x; i0 < n; i0 += 4 * kBinBlock) {
+            double x[4], y[4];
+            bool use[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = min(i0 + u * kBinBlock, n - 1);
+                use[u] = i0 + u * kBinBlock < n && !(valid && !valid[i]);
+                x[u] = pts[(long long)i * stride];
+                y[u] = pts[(long long)i * stride + 1];
+                if (origin) { x[u] += origin[2 * i]; y[u] += origin[2 * i + 1]; }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (use[u])
+                    fn(i0 + u * kBinBlock, x[u], y[u], bin_index(y[u], cell, gh) * gw + bin_index(x[u], cell, gw));
+        }
+    };
+    each([&](int, double, double, int b) { atomicAdd(&count[b], 1); });
+    __syncthreads();
+    // Exclusive scan of the counters in place, a run of consecutive ones per thread.
+    const int per = (bins + kBinBlock) / kBinBlock, b0 = threadIdx.x * per, b1 = min(b0 + per, bins + 1);
+    int acc = 0;
+    for (int b = b0; b < b1; ++b) acc += count[b];
+    int incl = acc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    const int w = warp_sums[lane];
+    int before = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += u;
+    }
+    int off = __shfl_sync(0xffffffffu, before - w, warp) + incl - acc;
+    for (int b = b0; b < b1; ++b) {
+        const int c = count[b];
+        start[b] = count[b] = off;
+        off += c;
+    }
+    __syncthreads();
+    each([&](int i, double x, double y, int b) {
+        const int slot = atomicAdd(&count[b], 1);
+        xy[slot] = make_double2(x, y);
+        id[slot] = i;
+    });
+}
+
+// Up to 8192 bins and 16384 points: one launch instead of seven operations (1,000 points in 1,024 bins: 4.9 us
+// against 17 us and their gaps; at 10,000 points both take some 15 us, and six launches less).
 int bin_build(BinStorage& b, const double* pts, int stride, const int* origin, const uint8_t* valid,
               long long n, cudaStream_t s) {
     const long long bins = (long long)b.gw * b.gh;
+    if (bins <= kBinsOneBlock && n <= kPointsOneBlock) {
+        k_bin_build_small<<<1, kBinBlock, (size_t)(bins + 1) * sizeof(int), s>>>(pts, stride, origin, valid, (int)n, b.gw,
+                                                                                b.gh, b.cell, b.start, b.xy, b.id);
+        return check_launch("k_bin_build_small");
+    }
     SPX_CUDA(cudaMemsetAsync(b.counts, 0, (bins + 1) * sizeof(int), s));
     SPX_CUDA(cudaMemsetAsync(b.fill, 0, (bins + 1) * sizeof(int), s));
     if (n > 0) {
