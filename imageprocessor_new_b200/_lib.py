@@ -78,6 +78,7 @@ SIGNATURES = {
     "spx_version": (_I, []),
     "spx_launch_count": (ctypes.c_ulonglong, []),
     "spx_device_info": (_I, [POINTER(c_int), POINTER(c_int)]),
+    "spx_download": (_I, [_P, _P, _S, _P, _S, _S, _I, _P]),
     "spx_fp64_fma_rate": (_I, [_I, _I, _P, POINTER(c_double), _P]),
     "spx_otsu_workspace_bytes": (_S, [_I]),
     "spx_otsu": (_I, [_P, _I, _I, _I, _I, _P, _P, _S, _P]),

@@ -691,10 +691,14 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
         seconds["result"] = time.perf_counter() - start
         seconds["total"] = time.perf_counter() - started
         return result
-    vor = c.voronoi.cpu().numpy()
-    remap = np.full(len(rows) + 1, -1, dtype=np.int32)
+    # The reported cells' labels and areas on the device, from the Voronoi labels of all cells.
+    remap = np.full(max(len(rows), 1), -1, dtype=np.int32)
     remap[report] = np.arange(nr, dtype=np.int32)
-    cell_labels = remap[vor]
+    remap_d = dev.upload(remap)
+    flat = c.voronoi.view(-1)
+    labels_out = remap_d.index_select(0, flat) if len(rows) else torch.full_like(flat, -1)
+    areas = torch.bincount(labels_out.add(1), minlength=nr + 1)[1:].cpu().numpy()
+    cell_labels = dev.download(labels_out.view(shape))
     params_global = state.params.copy()
     params_global[:, 1:3] += c.origins
     deblend_model = {"params": params_global, "report": report.astype(np.int64), "tile_px": int(state.tile_px)}
@@ -703,17 +707,17 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
     if metrics_only:
         rois, masks = np.empty((nr, 0, 0)), np.empty((nr, 0, 0), bool)
     else:
-        rois = cleaned.cpu().numpy()
+        rois = dev.download(cleaned)
         masks = _mask_stack(c, report)
     result = CDResult(
-        image=img_d.cpu().numpy() if isinstance(img, torch.Tensor) else img.copy(),
-        binary=np.zeros(shape, bool) if comp is None else comp.labels.cpu().numpy() > 0,
-        component_labels=np.zeros(shape, np.int32) if comp is None else comp.labels.cpu().numpy(),
+        image=dev.download(img_d) if isinstance(img, torch.Tensor) else img.copy(),
+        binary=np.zeros(shape, bool) if comp is None else dev.download(comp.labels > 0),
+        component_labels=np.zeros(shape, np.int32) if comp is None else dev.download(comp.labels),
         component_ids=np.asarray(component_ids, dtype=np.int32)[report],
         boxes_xywh=rows[report, :4].astype(np.int32), seeds_xy=c.seeds[report], cell_labels=cell_labels,
-        cell_areas_px2=np.bincount(cell_labels[cell_labels >= 0], minlength=nr), origins_xy=c.origins[report],
+        cell_areas_px2=areas, origins_xy=c.origins[report],
         rois=rois, masks=masks, measurements=measurements, pixel_size=float(pixel_size), unit=unit,
-        background_map=sign * state.background.host_map(), deblend_model=deblend_model, meta=meta,
+        background_map=state.background.host_map(sign), deblend_model=deblend_model, meta=meta,
     )
     seconds["result"] = time.perf_counter() - start
     seconds["total"] = time.perf_counter() - started
@@ -730,7 +734,7 @@ def _mask_stack(c, report) -> np.ndarray:
     inside = (r[None] < boxes[:, 3:4])[:, :, None] & (col[None] < boxes[:, 2:3])[:, None, :]
     ys = torch.clamp(boxes[:, 1:2] + r[None], 0, h - 1)[:, :, None]
     xs = torch.clamp(boxes[:, 0:1] + col[None], 0, w - 1)[:, None, :]
-    return (inside & (c.voronoi.to(torch.int64)[ys, xs] == rep[:, None, None])).cpu().numpy()
+    return dev.download(inside & (c.voronoi.to(torch.int64)[ys, xs] == rep[:, None, None]))
 
 
 _TAIL_CHUNK_BYTES = 512 * 2**20  # window arrays (float32 share + three byte masks) per chunk of holes

@@ -238,18 +238,18 @@ class Background:
         return _lib.BgMap(self.rows.data_ptr(), _ptr(self.j1), _ptr(self.t), self.ny, self.shape[1], 0.0,
                           _lib.BG_MAP)
 
-    def host_map(self) -> np.ndarray:
-        """The (H, W) map (subpx _upsample_tiles), built on the device and copied back."""
+    def host_map(self, sign: float = 1.0) -> np.ndarray:
+        """sign times the (H, W) map (subpx _upsample_tiles), built on the device and copied back."""
         h, w = self.shape
         if self.fixed is not None:
-            return np.full(self.shape, self.fixed)
+            return sign * np.full(self.shape, self.fixed)
         img = torch.zeros((h, w), dtype=torch.uint8, device="cuda")  # residual of a zero image = -bg
         model = torch.zeros((h, w), dtype=torch.float64, device="cuda")
         out = dev.empty((h, w), torch.float64)
         bg = self.struct()
         _lib.call("spx_residual", img.data_ptr(), 0, 1.0, h, w, bg, model.data_ptr(), out.data_ptr(),
                   dev.stream_ptr())
-        return -out.cpu().numpy()
+        return dev.download(out.neg_().mul_(sign))
 
     def at_points(self, xy_d: torch.Tensor, sign: float = 1.0) -> np.ndarray:
         """sign * map_coordinates(map, [y, x], order=1, mode="nearest") at device points (N, 2) [x, y]."""
@@ -340,12 +340,13 @@ class Deblender:
         h, w = self.shape
         tile = self.tile if tile is None else tile
         ny, nx = -(-h // tile), -(-w // tile)
-        med = dev.empty((ny * nx,), torch.float64)
-        cnt = dev.empty((ny * nx,), torch.int64)
+        both = dev.empty((2, ny * nx), torch.float64)  # medians, then counts (int64): one download
+        med, cnt = both[0], both[1].view(torch.int64)
         _lib.call("spx_tile_medians", self.img.data_ptr(), self.dtype, self.sign, h, w, _ptr(model),
                   _ptr(self.dist2), _ptr(self.usable_d), mode, float(thr_model), float(thr_dist), int(tile),
                   med.data_ptr(), cnt.data_ptr(), dev.stream_ptr())
-        return med.cpu().numpy().reshape(ny, nx), cnt.cpu().numpy().reshape(ny, nx)
+        host = both.cpu().numpy()
+        return host[0].reshape(ny, nx), host[1].view(np.int64).reshape(ny, nx)
 
     def stats(self, params_d, status_d, maxstep_d=None):
         """Median amplitude and FWHM of the good cells (subpx/_cpu/deblend.py:463-464) and, given the

@@ -97,7 +97,7 @@ def connected_components_stats(mask: np.ndarray, *, backend: str = "auto", conne
     with dev.on_device(device):
         comp = label(dev.upload(m), fixed_threshold=0.0, connectivity=connectivity)
         return ComponentStatsResult(
-            labels=comp.labels.cpu().numpy(), stats=comp.stats.cpu().numpy(),
-            centroids=comp.centroids.cpu().numpy(), num_labels=comp.count + 1, backend="gpu",
+            labels=dev.download(comp.labels), stats=dev.download(comp.stats),
+            centroids=dev.download(comp.centroids), num_labels=comp.count + 1, backend="gpu",
             meta={"connectivity": int(connectivity), "implementation": "libsubpx_b200 union-find CCL"},
         )

@@ -29,12 +29,11 @@ def dedupe_centers(centers_xy, *, eps: float = 1.5, device: int = 0) -> np.ndarr
     if len(pts) == 0:
         return pts
     with dev.on_device(device):
-        return _dedupe_device(dev.upload(pts), len(pts), float(eps)).cpu().numpy()
+        return dev.download(_dedupe_device(dev.upload(pts), len(pts), float(eps)))
 
 
 def _dedupe_device(pts_d: torch.Tensor, n: int, eps: float) -> torch.Tensor:
-    lo = pts_d.min(dim=0).values.cpu().numpy()
-    hi = pts_d.max(dim=0).values.cpu().numpy()
+    lo, hi = torch.stack(torch.aminmax(pts_d, dim=0)).cpu().numpy()
     args = (float(lo[0]), float(lo[1]), float(hi[0]), float(hi[1]), float(eps))
     ws = dev.workspace(_lib.size("spx_dedupe_workspace_bytes", n, *args))
     out = dev.empty((n, 2), torch.float64)
@@ -215,7 +214,7 @@ def detect_tiled(img, *, threshold, invert, area_min, area_max, pad, refine, con
         out = _keep_bands(bands, sum(len(c) for c, *_ in bands))
     kept, count = out
     n = dev.read_int(count)
-    centers = _dedupe_device(kept[:n].contiguous(), n, float(dedupe_eps)).cpu().numpy() if n else np.zeros((0, 2))
+    centers = dev.download(_dedupe_device(kept[:n].contiguous(), n, float(dedupe_eps))) if n else np.zeros((0, 2))
     meta = {"tile_h": int(tile_h), "overlap": int(overlap), "threshold_mode": str(threshold_mode),
             "band_graphs": bool(graphed),
             "otsu_downsample": int(otsu_downsample), "thr_scale": float(thr_scale), "dedupe_eps": float(dedupe_eps),

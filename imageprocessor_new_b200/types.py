@@ -76,11 +76,12 @@ class CDResult:
 
     def __post_init__(self):
         """Mean original intensity over each full Voronoi cell, without fill."""
-        assigned = self.cell_labels >= 0
+        # Bin 0 takes the pixels of no cell (label -1): the sums of the others run over the same pixels in the
+        # same order as over the assigned ones alone, without gathering them.
+        labels = np.asarray(self.cell_labels)
         totals = np.bincount(
-            self.cell_labels[assigned], weights=self.image[assigned].astype(np.float64),
-            minlength=len(self.seeds_xy),
-        )
+            (labels + 1).ravel(), weights=np.asarray(self.image, dtype=np.float64).ravel(), minlength=len(self.seeds_xy) + 1,
+        )[1:]
         self.mean_intensity = np.divide(
             totals, self.cell_areas_px2,
             out=np.full(len(self.seeds_xy), np.nan), where=self.cell_areas_px2 > 0,

@@ -29,7 +29,7 @@ def compute_voronoi_labels(seeds_xy: np.ndarray, image_shape, *, device: int = 0
     seeds = seeds.reshape(-1, 2)
     with dev.on_device(device):
         sd = dev.upload(seeds) if len(seeds) else None
-        return labels_device(sd, image_shape).cpu().numpy()
+        return dev.download(labels_device(sd, image_shape))
 
 
 compute_voronoi_labels_gpu = compute_voronoi_labels

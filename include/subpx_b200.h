@@ -67,6 +67,12 @@ int spx_tune_set(const char* knob, int value);
 int spx_tune_get(const char* knob, int* value);
 /* Number of SMs of the current device, and whether it is an sm_100 part (1) or not (0). */
 int spx_device_info(int* sm_count, int* is_sm100);
+/* Copies bytes of device memory to ordinary (pageable) host memory, in chunks through the caller's
+ * page-locked buffer (pinned_bytes / chunk slots, at most 16), copied out by up to `threads` host threads
+ * (at most 8) of this call while later chunks arrive. Ordered after the work queued on the stream; returns
+ * when dst is complete. */
+int spx_download(void* dst, const void* src, size_t bytes, void* pinned, size_t pinned_bytes, size_t chunk, int threads,
+                 void* stream);
 /* FP64 FMA throughput probe (no reference counterpart): `blocks` x 256 threads each run eight
  * independent FP64 FMA chains of `iters` steps; *flops (host) = the launch's floating-point
  * operations (2 per FMA), so that a caller timing the launch gets the device's FP64 rate, the
