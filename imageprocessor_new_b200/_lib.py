@@ -115,6 +115,7 @@ SIGNATURES = {
     "spx_status_name": (ctypes.c_char_p, [_I]),
     "spx_status_text": (_I, [_P, _I, _P, _P]),
     "spx_refine_centers_counted": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _I, _I, _P, _P]),
+    "spx_refine_selected": (_I, [_P, _I, _I, _I, _P, _P, _P, _I, _P, _I, _I, _P, _P]),
     "spx_refine_centers": (_I, [_P, _I, _I, _I, _P, _P, _P, _I, _I, _P, _P]),
     "spx_keep_band_workspace_bytes": (_S, [_I]),
     "spx_keep_band": (_I, [_P, _I, _D, _D, _D, _P, _P, _I, _P, _S, _P]),

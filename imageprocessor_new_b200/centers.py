@@ -96,8 +96,9 @@ def _centers_on_device(img_d: torch.Tensor, *, threshold_dev: torch.Tensor | Non
               kept.data_ptr(), ws.data_ptr(), ws.numel(), dev.stream_ptr())
     n = dev.read_int(kept)
     centers = dev.empty((max(n, 1), 2), torch.float64)
-    _lib.call("spx_refine_centers", img_d.data_ptr(), dev.dtype_code(img_d), h, w, comp.labels.data_ptr(),
-              rows.data_ptr(), methods.data_ptr(), n, int(pad), centers.data_ptr(), dev.stream_ptr())
+    _lib.call("spx_refine_selected", img_d.data_ptr(), dev.dtype_code(img_d), h, w, comp.labels.data_ptr(),
+              rows.data_ptr(), methods.data_ptr(), n, None, int(pad), _lib.REFINE_CODES[refine], centers.data_ptr(),
+              dev.stream_ptr())
     return centers[:n]
 
 
@@ -227,8 +228,9 @@ def _deblended_cells_centers(img_d: torch.Tensor, sign: float, seeds: np.ndarray
               state.params_d.data_ptr(), n, hm, wm, w, labels.data_ptr(), refine_rows.data_ptr(), stream)
     methods = torch.full((n,), _lib.REFINE_CODES[refine], dtype=torch.uint8, device="cuda")
     local = dev.empty((n, 2), torch.float64)
-    _lib.call("spx_refine_centers", cleaned.data_ptr(), _lib.DTYPES[np.dtype(np.float64)], n * hm, wm,
-              labels.data_ptr(), refine_rows.data_ptr(), methods.data_ptr(), n, 0, local.data_ptr(), stream)
+    _lib.call("spx_refine_selected", cleaned.data_ptr(), _lib.DTYPES[np.dtype(np.float64)], n * hm, wm,
+              labels.data_ptr(), refine_rows.data_ptr(), methods.data_ptr(), n, None, 0, _lib.REFINE_CODES[refine],
+              local.data_ptr(), stream)
     centres = local.cpu().numpy()
     centres[:, 1] -= np.arange(n) * hm  # window row -> cell row
     centres += cells.origins

@@ -188,6 +188,11 @@ int spx_refine_centers(const void* img, int dtype, int height, int width, const 
 int spx_refine_centers_counted(const void* img, int dtype, int height, int width, const int* labels,
                                const int* rows, const uint8_t* methods, const int* n_dev, int capacity, int pad,
                                double* centers_out, void* stream);
+/* The same for rows and methods that spx_select_components wrote for `refine`: launches only the refiners
+ * it can have chosen. n_dev (optional): the device count of live rows among n, the rest NaN. */
+int spx_refine_selected(const void* img, int dtype, int height, int width, const int* labels, const int* rows,
+                        const uint8_t* methods, int n, const int* n_dev, int pad, int refine, double* centers_out,
+                        void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Tiled detection (detect_centers(tile_h=...), subpx/_gpu/centers.py:1778-1862 and

@@ -1,0 +1,87 @@
+"""The refiners on integer images (ROIs up to 32 x 32 px staged in shared memory) against the same
+refiners on the same image as float64, which takes the general path: blob sizes on either side of 16 and
+32 px ROIs, one-pixel and two-pixel-thick blobs, ROIs clipped by the image, masks that are not their box.
+
+Weighted centroids, mask means and edges are sums of exact terms or per-pixel arithmetic: the same bits.
+The log-quadratic normal equations are sums in another order: 1e-9 px, the refiners' own tolerance."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (1, 2, 3, 8, 10, 11, 12, 25, 26, 27, 40)
+
+
+def _scene(dtype, seed):
+    rng = np.random.default_rng(seed)
+    top = 250 if dtype == "uint8" else 4000
+    boxes, y = [], 0
+    for k, h in enumerate(SIZES):
+        x = 0 if k % 3 == 0 else 5
+        for w in SIZES:
+            boxes.append((x, y, w, h))
+            x += w + 9
+        y += h + 9
+    hgt, wid = y - 9 + (1 if seed else 0), max(x + w for x, _, w, _ in boxes)
+    img = rng.normal(0.2 * top, 0.01 * top, (hgt, wid))
+    labels = np.zeros((hgt, wid), np.int32)
+    rows = []
+    for k, (x, y, w, h) in enumerate(boxes):
+        yy, xx = np.mgrid[:h, :w]
+        cy, cx = (h - 1) / 2 + rng.uniform(-0.3, 0.3), (w - 1) / 2 + rng.uniform(-0.3, 0.3)
+        r2 = ((yy - cy) / max(0.5 * h, 0.7)) ** 2 + ((xx - cx) / max(0.5 * w, 0.7)) ** 2
+        m = r2 <= 1.3
+        m[int(round(cy)), int(round(cx))] = True
+        img[y:y + h, x:x + w] += 0.7 * top * np.exp(-0.5 * r2)
+        labels[y:y + h, x:x + w][m] = k + 1
+        rows.append((x, y, w, h, k + 1))
+    return np.clip(np.rint(img), 0, top * 1.02).astype(dtype), labels, np.array(rows, np.int32)
+
+
+@pytest.mark.parametrize("dtype", ["uint8", "uint16"])
+@pytest.mark.parametrize("refine", ["none", "weighted", "logquad", "edge_gradmoment"])
+@pytest.mark.parametrize("pad", [0, 3])
+def test_staged_rois_match_the_general_path(dtype, refine, pad):
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    for seed in (0, 1):
+        img, labels, rows = _scene(dtype, seed)
+        n, code = len(rows), _lib.REFINE_CODES[refine]
+        lab_d, rows_d = dev.upload(labels), dev.upload(rows)
+        meth_d = dev.upload(np.full(n, code, np.uint8))
+        got = []
+        for image in (img, img.astype(np.float64)):
+            img_d, out = dev.upload(image), dev.upload(np.zeros((n, 2)))
+            _lib.call("spx_refine_selected", img_d.data_ptr(), dev.dtype_code(img_d), *labels.shape, lab_d.data_ptr(),
+                      rows_d.data_ptr(), meth_d.data_ptr(), n, None, pad, code, out.data_ptr(), dev.stream_ptr())
+            both = dev.upload(np.zeros((n, 2)))
+            _lib.call("spx_refine_centers", img_d.data_ptr(), dev.dtype_code(img_d), *labels.shape, lab_d.data_ptr(),
+                      rows_d.data_ptr(), meth_d.data_ptr(), n, pad, both.data_ptr(), dev.stream_ptr())
+            got.append(out.cpu().numpy())
+            np.testing.assert_array_equal(both.cpu().numpy(), got[-1])
+        assert np.isfinite(got[0]).all(axis=1).mean() > 0.3
+        if refine == "logquad":
+            np.testing.assert_allclose(got[0], got[1], rtol=0, atol=1e-9)
+        else:
+            np.testing.assert_array_equal(got[0], got[1])
+
+
+def test_rows_past_a_device_count_are_nan():
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    img, labels, rows = _scene("uint16", 0)
+    n = len(rows)
+    img_d, lab_d, rows_d = dev.upload(img), dev.upload(labels), dev.upload(rows)
+    live = dev.upload(np.array([n // 2], np.int32))
+    for refine in ("weighted", "logquad", "auto", "none"):
+        code = _lib.REFINE_CODES[refine]
+        meth = np.where(np.arange(n) % 2, 2, 3) if refine == "auto" else np.full(n, code)
+        meth_d, out = dev.upload(meth.astype(np.uint8)), dev.upload(np.full((n, 2), -7.0))  # -7: not written
+        _lib.call("spx_refine_selected", img_d.data_ptr(), dev.dtype_code(img_d), *labels.shape, lab_d.data_ptr(),
+                  rows_d.data_ptr(), meth_d.data_ptr(), n, live.data_ptr(), 3, code, out.data_ptr(), dev.stream_ptr())
+        c = out.cpu().numpy()
+        assert np.isnan(c[n // 2:]).all()
+        assert np.isfinite(c[: n // 2]).any() and not (c == -7.0).any()
