@@ -5,13 +5,18 @@ in place of the reference's O(N^2) Python loop.
 
 With the global threshold, each band's pipeline (binarise, optional open / close, CCL, area filter,
 refiners) is captured once as a CUDA graph over fixed buffers and replayed for every band of the
-same height: the band is copied into the graph's input buffer, the counts stay on the device (the
+same height, on this page and on later ones: the band is copied into the graph's input buffer and the
+page's threshold into its threshold (both stay on the device), the counts stay on the device (the
 refiners run over a fixed capacity of rows, those past the selected count giving NaN centres that
 the keep rule drops), and the host reads the per-band component counts once at the end. The
 capacity is twice the components of the band the graph was built on; a page with a band of more
-components than that is redone by the eager path (and the graph rebuilt on the next call)."""
+components than that is redone by the eager path (and the graph rebuilt, for that many, on the next
+call). Idle graphs wait in a small pool; a call takes the ones it uses out of it and puts them back
+once its work has finished, so calls from several threads or on several streams never share one."""
 
 from __future__ import annotations
+
+import threading
 
 import numpy as np
 import torch
@@ -57,10 +62,10 @@ def band_capacity(band_h: int, width: int, components: int | None = None) -> int
 class BandGraph:
     """The per-band pipeline of one band height, captured as a CUDA graph (see the module docstring)."""
 
-    def __init__(self, band_h: int, width: int, dtype: torch.dtype, *, fixed_threshold: float, invert: bool,
+    def __init__(self, band_h: int, width: int, dtype: torch.dtype, *, threshold: torch.Tensor, invert: bool,
                  area_min: int, area_max: int, pad: int, refine: str, connectivity: int, small_feature_max: float,
                  morph_open: int = 0, morph_close: int = 0, capacity: int | None = None,
-                 sample: torch.Tensor | None = None):
+                 sample: torch.Tensor | None = None, components: int = 0):
         from .centers import _segmentation_source
 
         self.shape = (int(band_h), int(width))
@@ -71,15 +76,16 @@ class BandGraph:
         self.kept = torch.zeros(1, dtype=torch.int32, device="cuda")
         self.ccl_ws = dev.workspace(_lib.size("spx_ccl_workspace_bytes", h, w))
         self._seg = _segmentation_source
-        self._seg_args = (float(fixed_threshold), bool(invert), int(morph_open), int(morph_close))
+        self._seg_args = (bool(invert), int(morph_open), int(morph_close))
+        self.threshold = threshold.clone()  # the page's, one device double
         if capacity is None and sample is not None:
             # Size the capacity on a real band: its component count, from the labelling alone.
             self.src.copy_(sample)
-            src, thr, fixed, inv = self._seg(self.src, None, *self._seg_args)
+            src, thr, fixed, inv = self._seg(self.src, self.threshold, 0.0, *self._seg_args)
             _lib.call("spx_ccl_label", src.data_ptr(), dev.dtype_code(src), h, w, dev.ptr(thr), float(fixed),
                       int(bool(inv)), int(connectivity), self.labels.data_ptr(), self.count.data_ptr(),
                       self.ccl_ws.data_ptr(), self.ccl_ws.numel(), dev.stream_ptr())
-            capacity = band_capacity(h, w, dev.read_int(self.count))
+            capacity = band_capacity(h, w, max(int(components), dev.read_int(self.count)))
         self.capacity = int(capacity) if capacity is not None else band_capacity(h, w)
         cap = self.capacity
         self.stats = dev.empty((cap + 1, 5), torch.int32)
@@ -99,8 +105,7 @@ class BandGraph:
     def _launch(self):
         h, w = self.shape
         area_min, area_max, pad, refine, conn, sfm = self._params
-        fixed, invert, mo, mc = self._seg_args
-        src, thr, fixed, inv = self._seg(self.src, None, fixed, invert, mo, mc)
+        src, thr, fixed, inv = self._seg(self.src, self.threshold, 0.0, *self._seg_args)
         stream = dev.stream_ptr()
         _lib.call("spx_ccl_label", src.data_ptr(), dev.dtype_code(src), h, w, dev.ptr(thr), float(fixed),
                   int(bool(inv)), conn, self.labels.data_ptr(), self.count.data_ptr(), self.ccl_ws.data_ptr(),
@@ -112,19 +117,36 @@ class BandGraph:
         _lib.call("spx_select_components", self.stats.data_ptr(), self.capacity, area_min, area_max, refine, sfm,
                   self.rows.data_ptr(), self.methods.data_ptr(), self.kept.data_ptr(), self.sel_ws.data_ptr(),
                   self.sel_ws.numel(), stream)
-        _lib.call("spx_refine_centers_counted", self.src.data_ptr(), dev.dtype_code(self.src), h, w,
-                  self.labels.data_ptr(), self.rows.data_ptr(), self.methods.data_ptr(), self.kept.data_ptr(),
-                  self.capacity, pad, self.centers.data_ptr(), stream)
+        _lib.call("spx_refine_selected", self.src.data_ptr(), dev.dtype_code(self.src), h, w,
+                  self.labels.data_ptr(), self.rows.data_ptr(), self.methods.data_ptr(), self.capacity,
+                  self.kept.data_ptr(), pad, refine, self.centers.data_ptr(), stream)
 
-    def run(self, band: torch.Tensor) -> torch.Tensor:
-        """Replays the pipeline on `band` (same shape); returns the (capacity, 2) centres (NaN rows
-        past the kept count) and leaves the band's component count in self.count."""
+    def run(self, band: torch.Tensor, threshold: torch.Tensor) -> torch.Tensor:
+        """Replays the pipeline on `band` (same shape) at a device threshold; returns the (capacity, 2)
+        centres (NaN rows past the kept count) and leaves the band's component count in self.count."""
         self.src.copy_(band)
+        self.threshold.copy_(threshold)
         self.graph.replay()
         return self.centers
 
 
-_GRAPHS: dict = {}
+_GRAPHS: dict = {}      # key -> idle graphs of that key
+_COMPONENTS: dict = {}  # key -> components of the fullest band that overflowed a graph of that key
+_GRAPHS_MOST = 4        # idle graphs kept
+_GRAPHS_LOCK = threading.Lock()
+
+
+def _take_graph(key):
+    with _GRAPHS_LOCK:
+        idle = _GRAPHS.get(key)
+        return idle.pop() if idle else None
+
+
+def _put_graph(key, graph):
+    with _GRAPHS_LOCK:
+        if sum(len(v) for v in _GRAPHS.values()) >= _GRAPHS_MOST:
+            _GRAPHS.clear()
+        _GRAPHS.setdefault(key, []).append(graph)
 
 
 def _keep_bands(bands, kept_rows):
@@ -139,35 +161,46 @@ def _keep_bands(bands, kept_rows):
     return kept, count
 
 
-def _bands_with_graphs(img_d, spans, pre, common):
-    """Every band through a cached BandGraph of its height; None when a band overflows its capacity."""
+def _bands_with_graphs(img_d, spans, thr, common):
+    """Every band through a BandGraph of its height at the device threshold; None when a band overflows
+    its capacity."""
     width = img_d.shape[1]
-    graphs = {}
-    keys = {}
+    graphs = {}  # band height -> (key, graph), this call's own until they are put back
     for y0, y1, _, _ in spans:
-        key = (y1 - y0, width, img_d.dtype, float(pre), tuple(sorted(common.items())), torch.cuda.current_device(),
+        if y1 - y0 in graphs:
+            continue
+        key = (y1 - y0, width, img_d.dtype, tuple(sorted(common.items())), torch.cuda.current_device(),
                BAND_PX_PER_COMPONENT)
-        if key not in _GRAPHS:
-            if len(_GRAPHS) >= 4:
-                _GRAPHS.clear()
-            _GRAPHS[key] = BandGraph(y1 - y0, width, img_d.dtype, fixed_threshold=pre, sample=img_d[y0:y1],
-                                     **common)
-        graphs[(y0, y1)] = _GRAPHS[key]
-        keys[(y0, y1)] = key
-    cap_total = sum(graphs[(y0, y1)].capacity for y0, y1, _, _ in spans)
+        graph = _take_graph(key)
+        if graph is None:
+            graph = BandGraph(y1 - y0, width, img_d.dtype, threshold=thr, sample=img_d[y0:y1],
+                              components=_COMPONENTS.get(key, 0), **common)
+        graphs[y1 - y0] = (key, graph)
+    cap_total = sum(graphs[y1 - y0][1].capacity for y0, y1, _, _ in spans)
     kept = dev.empty((max(cap_total, 1), 2), torch.float64)
     count = torch.zeros(1, dtype=torch.int32, device="cuda")
     counts = torch.zeros(len(spans), dtype=torch.int32, device="cuda")
-    ws = dev.workspace(_lib.size("spx_keep_band_workspace_bytes", max(g.capacity for g in graphs.values())))
+    ws = dev.workspace(_lib.size("spx_keep_band_workspace_bytes", max(g.capacity for _, g in graphs.values())))
     for b, (y0, y1, lo, hi) in enumerate(spans):
-        g = graphs[(y0, y1)]
-        centers = g.run(img_d[y0:y1])
+        g = graphs[y1 - y0][1]
+        centers = g.run(img_d[y0:y1], thr)
         counts[b:b + 1].copy_(g.count)
         _lib.call("spx_keep_band", centers.data_ptr(), g.capacity, float(y0), float(lo), float(hi), kept.data_ptr(),
                   count.data_ptr(), max(cap_total, 1), ws.data_ptr(), ws.numel(), dev.stream_ptr())
-    over = [b for b, c in enumerate(counts.cpu().numpy()) if int(c) > graphs[spans[b][:2]].capacity]
-    for b in over:  # rebuilt on the next call, sized on a band of this page
-        _GRAPHS.pop(keys[spans[b][:2]], None)
+    found = counts.cpu().numpy()  # (the graphs' work has finished)
+    over = set()
+    for (y0, y1, _, _), c in zip(spans, found):
+        if int(c) > graphs[y1 - y0][1].capacity:  # rebuilt for that many on the next call
+            over.add(y1 - y0)
+            key = graphs[y1 - y0][0]
+            with _GRAPHS_LOCK:
+                if len(_COMPONENTS) >= 64 and key not in _COMPONENTS:
+                    _COMPONENTS.clear()
+                _COMPONENTS[key] = max(_COMPONENTS.get(key, 0), int(c))
+                _GRAPHS.pop(key, None)
+    for height, (key, graph) in graphs.items():
+        if height not in over:
+            _put_graph(key, graph)
     return None if over else (kept, count)
 
 
@@ -182,10 +215,9 @@ def detect_tiled(img, *, threshold, invert, area_min, area_max, pad, refine, con
         raise ValueError("threshold_mode must be 'auto', 'global' or 'per_tile'")
     img_d = _device_image(img)
     height, width = img_d.shape
-    pre = None
+    pre = None  # the global threshold, one device double
     if threshold_mode in ("global", "auto"):
-        ds = max(1, int(otsu_downsample))
-        pre = float(segment.otsu(img_d, step=ds).item()) * float(thr_scale)
+        pre = segment.otsu(img_d, step=max(1, int(otsu_downsample))).mul_(float(thr_scale))
     step = tile_h - overlap
     spans = []
     y0 = 0
@@ -208,8 +240,8 @@ def detect_tiled(img, *, threshold, invert, area_min, area_max, pad, refine, con
         bands = []
         for y0, y1, lo, hi in spans:
             band = img_d[y0:y1]
-            thr = segment.binarize_threshold(band, threshold, invert) if pre is None else None
-            c = _centers_on_device(band, threshold_dev=thr, fixed_threshold=pre if pre is not None else 0.0, **common)
+            thr = segment.binarize_threshold(band, threshold, invert) if pre is None else pre
+            c = _centers_on_device(band, threshold_dev=thr, fixed_threshold=0.0, **common)
             bands.append((c, y0, lo, hi))
         out = _keep_bands(bands, sum(len(c) for c, *_ in bands))
     kept, count = out
