@@ -96,7 +96,7 @@ int spx_otsu(const void* img, int dtype, int height, int width, int step, double
  * workspace: code running inside CUDA stream capture or a real-time acquisition loop, where
  * cudaMalloc would synchronise the device or fail under a fixed memory budget, and hosts whose own
  * allocator owns every device byte. No counterpart in the reference: it is spx_otsu with its scratch
- * in a 2.3 MiB file-scope device array that every GPU loading the library holds until exit.
+ * in a 0.25 MiB file-scope device array that every GPU loading the library holds until exit.
  * Limit: at most 4294967295 sampled pixels (ceil(H/step) * ceil(W/step)), the range of the 32-bit
  * histogram counts; larger images are rejected with SPX_ERR_ARGUMENT. The first call on a device
  * looks up the array's device address (cudaGetSymbolAddress), so make it before any stream capture;
