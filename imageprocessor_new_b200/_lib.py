@@ -138,6 +138,8 @@ SIGNATURES = {
     "spx_cell_stats": (_I, [_P, _P, _I, _P, _P, _P]),
     "spx_background_at": (_I, [_BG, _I, _I, _P, _I, _D, _P, _P]),
     "spx_clean_cells": (_I, [_P, _I, _D, _I, _I, _P, _P, _P, _I, _BG, _P, _P, _I, _I, _I, _P, _P]),
+    "spx_deblend_measure_workspace_bytes": (_S, [_I]),
+    "spx_deblend_measure": (_I, [_P, _I, _D, _I, _I, _P, _P, _P, _P, _P, _P, _I, _D, _D, _I, _I, _P, _P, _S, _P]),
     "spx_tile_medians": (_I, [_P, _I, _D, _I, _I, _P, _P, _P, _I, _D, _D, _I, _P, _P, _P]),
     "spx_background_rows": (_I, [_P, _I, _I, _I, _I, _P, _P]),
     "spx_residual": (_I, [_P, _I, _D, _I, _I, _BG, _P, _P, _P]),

@@ -743,6 +743,18 @@ __global__ void k_support_labels(const double* cleaned, const int* vor, const in
 
 // ------------------------------------------------------------------------------ tile medians
 
+// Smallest integer squared distance whose square root reaches thr_dist (sqrt is correctly rounded on the host
+// and on the device, and monotonic), so that the kernel compares integers.
+__host__ __device__ inline unsigned long long distance_floor(double thr_dist) {
+    if (thr_dist != thr_dist) return 1ull << 33;  // NaN: no distance passes
+    if (!(thr_dist > 0.0)) return 0;
+    const double t2 = ceil(thr_dist * thr_dist);
+    unsigned long long d = t2 > 8.0e9 ? (1ull << 33) : (unsigned long long)t2;
+    while (d > 0 && sqrt((double)(d - 1)) >= thr_dist) --d;
+    while (d < (1ull << 33) && !(sqrt((double)d) >= thr_dist)) ++d;
+    return d;
+}
+
 constexpr int kTileThreads = 512;
 constexpr int kTileSmemKeys = 24576;  // keys held in shared memory (192 KiB)
 
@@ -753,7 +765,11 @@ struct TileSel {
     const uint8_t* usable;    // null: all usable
     int mode;                 // SPX_TILE_FREE: model < thr_model & dist >= thr_dist; SPX_TILE_USABLE; SPX_TILE_ALL
     double thr_model;
-    unsigned long long d2_min;  // sqrt((double)d2) >= thr_dist  <=>  d2 >= d2_min (set by the host)
+    unsigned long long d2_min;  // sqrt((double)d2) >= thr_dist  <=>  d2 >= d2_min (distance_floor)
+    // When stats is given (SPX_TILE_FREE): thr_model = frac * median amplitude and thr_dist = mult * median FWHM of
+    // the good cells, (value, count) pairs in stats; 1 and 0 when there are none.
+    const double* stats;
+    double frac, mult;
     // A pixel's loads (pixel of type Px, model, distance, usable flag), none of them conditional on
     // another's value, so that a thread's loads of several pixels are in flight together.
     struct Loaded {
@@ -797,7 +813,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_tile_median(TileSel sel, in
     __shared__ int hist[2048];
     __shared__ int warp_tot[32], s_pick[3];
     __shared__ int s_count;
-    __shared__ unsigned long long s_keys[2], s_kmin, s_kmax;
+    __shared__ unsigned long long s_keys[2], s_kmin, s_kmax, s_floor;
     const int ty = blockIdx.x / nx, tx = blockIdx.x % nx;
     const int y0 = ty * tile, x0 = tx * tile;
     const int th = min(tile, sel.img.H - y0), tw = min(tile, sel.img.W - x0);
@@ -807,8 +823,13 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_tile_median(TileSel sel, in
         s_count = 0;
         s_kmin = ~0ull;
         s_kmax = 0;
+        if (sel.stats) s_floor = distance_floor(sel.mult * (sel.stats[3] > 0.0 ? sel.stats[2] : 0.0));
     }
     __syncthreads();
+    if (sel.stats) {
+        sel.thr_model = sel.frac * (sel.stats[1] > 0.0 ? sel.stats[0] : 1.0);
+        sel.d2_min = s_floor;
+    }
     // Pass 0: count and (when they fit) stage the keys, kPass0 pixels per thread at a time so
     // that their loads are in flight together. The loop bounds are the same for every thread, so
     // the warp votes are over full warps.
@@ -953,17 +974,16 @@ __device__ __forceinline__ bool q_select(const QuantileReq& r, int i, double* v)
 constexpr int kQuantThreads = 1024;
 constexpr int kQuantAhead = 4;
 
-// One CTA per request: out[2 * b] = result (NaN when nothing is selected), out[2 * b + 1] = count.
+// One CTA per request: out[0] = result (NaN when nothing is selected), out[1] = count.
 // A counting pass finds the count, whether a NaN is selected and the smallest and largest key;
 // cta_select then finds the order statistics, kQuantAhead values per thread loaded before their
 // histogram updates so that the loads overlap.
-__global__ void __launch_bounds__(kQuantThreads) k_quantiles(const QuantileReq* reqs, double* out) {
+__device__ __forceinline__ void cta_quantile(const QuantileReq& r, double* out) {
     __shared__ int hist[2048];
     __shared__ int warp_tot[32];
     __shared__ int s_pick[3];
     __shared__ int s_count, s_nan;
     __shared__ unsigned long long s_keys[2], s_kmin, s_kmax;
-    const QuantileReq r = reqs[blockIdx.x];
     if (threadIdx.x == 0) {
         s_count = s_nan = 0;
         s_kmin = ~0ull;
@@ -1032,9 +1052,23 @@ __global__ void __launch_bounds__(kQuantThreads) k_quantiles(const QuantileReq* 
         }
     }
     if (threadIdx.x == 0) {
-        out[2 * blockIdx.x] = res;
-        out[2 * blockIdx.x + 1] = (double)n;
+        out[0] = res;
+        out[1] = (double)n;
     }
+}
+
+__global__ void __launch_bounds__(kQuantThreads) k_quantiles(const QuantileReq* reqs, double* out) {
+    const QuantileReq r = reqs[blockIdx.x];
+    cta_quantile(r, out + 2 * blockIdx.x);
+}
+
+// k_quantiles with its requests among the launch arguments (no upload before it).
+struct CellQuantiles {
+    QuantileReq r[3];
+};
+__global__ void __launch_bounds__(kQuantThreads) k_cell_quantiles(CellQuantiles q, double* out) {
+    const QuantileReq r = q.r[blockIdx.x];
+    cta_quantile(r, out + 2 * blockIdx.x);
 }
 
 // Per-cell amplitude, 2 sqrt(2 ln 2) sigma_major and the "good" flag (status ok and A > 0).
@@ -1409,14 +1443,9 @@ int spx_support_labels(const double* cleaned, const int* voronoi, const int* box
     return check_launch("k_support_labels");
 }
 
-int spx_tile_medians(const void* img, int dtype, double sign, int height, int width, const double* model,
-                     const unsigned int* dist2, const uint8_t* usable, int mode, double thr_model, double thr_dist,
-                     int tile, double* medians, long long* counts, void* stream) {
-    SPX_REQUIRE(height > 0 && width > 0 && tile >= 1, "bad arguments");
-    SPX_REQUIRE(mode == SPX_TILE_FREE || mode == SPX_TILE_USABLE || mode == SPX_TILE_ALL, "bad mode");
-    SPX_REQUIRE(img && medians && counts && (mode != SPX_TILE_FREE || dist2), "null pointer");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int ny = (height + tile - 1) / tile, nx = (width + tile - 1) / tile;
+static int launch_tile_medians(const TileSel& sel, int dtype, int tile, double* medians, long long* counts,
+                               cudaStream_t s) {
+    const int ny = (sel.img.H + tile - 1) / tile, nx = (sel.img.W + tile - 1) / tile;
     const long long t2 = (long long)tile * tile;
     const int smem_keys = (int)(t2 < kTileSmemKeys ? t2 : kTileSmemKeys);
     const size_t smem = (size_t)smem_keys * sizeof(unsigned long long);
@@ -1424,21 +1453,58 @@ int spx_tile_medians(const void* img, int dtype, double sign, int height, int wi
                   : dtype == SPX_U16 ? k_tile_median<uint16_t>
                   : dtype == SPX_F32 ? k_tile_median<float> : k_tile_median<double>;
     SPX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // Smallest integer squared distance whose square root reaches thr_dist (sqrt is correctly
-    // rounded here and on the device, and monotonic), so the kernel compares integers.
-    unsigned long long d2_min = 0;
-    if (thr_dist != thr_dist) {
-        d2_min = 1ull << 33;  // NaN: no distance passes
-    } else if (thr_dist > 0.0) {
-        const double t2 = ceil(thr_dist * thr_dist);
-        unsigned long long d = t2 > 8.0e9 ? (1ull << 33) : (unsigned long long)t2;
-        while (d > 0 && sqrt((double)(d - 1)) >= thr_dist) --d;
-        while (d < (1ull << 33) && !(sqrt((double)d) >= thr_dist)) ++d;
-        d2_min = d;
-    }
-    TileSel sel{Image{img, dtype, sign, height, width}, model, dist2, usable, mode, thr_model, d2_min};
     kernel<<<ny * nx, kTileThreads, smem, s>>>(sel, tile, nx, smem_keys, medians, counts);
     return check_launch("k_tile_median");
+}
+
+int spx_tile_medians(const void* img, int dtype, double sign, int height, int width, const double* model,
+                     const unsigned int* dist2, const uint8_t* usable, int mode, double thr_model, double thr_dist,
+                     int tile, double* medians, long long* counts, void* stream) {
+    SPX_REQUIRE(height > 0 && width > 0 && tile >= 1, "bad arguments");
+    SPX_REQUIRE(mode == SPX_TILE_FREE || mode == SPX_TILE_USABLE || mode == SPX_TILE_ALL, "bad mode");
+    SPX_REQUIRE(img && medians && counts && (mode != SPX_TILE_FREE || dist2), "null pointer");
+    const TileSel sel{Image{img, dtype, sign, height, width}, model, dist2, usable, mode, thr_model,
+                      distance_floor(thr_dist), nullptr, 0.0, 0.0};
+    return launch_tile_medians(sel, dtype, tile, medians, counts, static_cast<cudaStream_t>(stream));
+}
+
+size_t spx_deblend_measure_workspace_bytes(int n) {
+    Arena a(nullptr);
+    a.take<double>(n > 0 ? n : 0);
+    a.take<uint8_t>(n > 0 ? n : 0);
+    return a.used;
+}
+
+int spx_deblend_measure(const void* img, int dtype, double sign, int height, int width, const double* model,
+                        const unsigned int* dist2, const uint8_t* usable, const double* params, const uint8_t* status,
+                        const double* maxstep, int n, double free_fraction, double free_distance_fwhm, int tile,
+                        int with_usable, double* out, void* workspace, size_t workspace_bytes, void* stream) {
+    SPX_REQUIRE(n >= 1 && tile >= 0 && height > 0 && width > 0, "bad arguments");
+    SPX_REQUIRE(params && status && out && workspace, "null pointer");
+    SPX_REQUIRE(tile == 0 || (img && model && dist2), "null pointer");
+    SPX_REQUIRE(workspace_bytes >= spx_deblend_measure_workspace_bytes(n), "workspace too small");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    Arena a(workspace);
+    double* fwhm = a.take<double>(n);
+    uint8_t* good = a.take<uint8_t>(n);
+    k_cell_stats<<<grid_for(n, 256), 256, 0, s>>>(params, status, n, fwhm, good);
+    if (int e = check_launch("k_cell_stats")) return e;
+    const CellQuantiles q{{{params, 6, good, 0, n, 0, 0.0},
+                           {fwhm, 1, good, 0, n, 0, 0.0},
+                           {maxstep, 1, nullptr, 1, maxstep ? n : 0, 1, 99.0 / 100.0}}};
+    k_cell_quantiles<<<3, kQuantThreads, 0, s>>>(q, out);
+    if (int e = check_launch("k_cell_quantiles")) return e;
+    if (tile == 0) return SPX_OK;
+    const long long tiles = (long long)((height + tile - 1) / tile) * ((width + tile - 1) / tile);
+    TileSel sel{Image{img, dtype, sign, height, width}, model, dist2, usable, SPX_TILE_FREE, 0.0, 0, out,
+                free_fraction, free_distance_fwhm};
+    double* at = out + 6;
+    if (int e = launch_tile_medians(sel, dtype, tile, at, reinterpret_cast<long long*>(at + tiles), s)) return e;
+    if (!with_usable) return SPX_OK;
+    sel.mode = SPX_TILE_USABLE;
+    sel.stats = nullptr;
+    at += 2 * tiles;
+    return launch_tile_medians(sel, dtype, tile, at, reinterpret_cast<long long*>(at + tiles), s);
 }
 
 int spx_background_rows(const double* medians, int ny, int nx, int tile, int width, double* rows, void* stream) {

@@ -313,6 +313,7 @@ class Deblender:
         self.radius_cap = int(max(cells.hm, cells.wm)) if self.n else 2
         self.fit_ws = dev.workspace(_lib.size("spx_fit_workspace_bytes", cells.max_px))
         self.render_ws = dev.workspace(_lib.size("spx_render_workspace_bytes", self.n, h, w))
+        self.measure_ws = dev.workspace(_lib.size("spx_deblend_measure_workspace_bytes", self.n))
         if self.n:
             _lib.call("spx_render_overflow", self.render_ws.data_ptr(), self.n, h, w, ctypes.byref(ctypes.c_int(0)), 1,
                       dev.stream_ptr())
@@ -363,30 +364,58 @@ class Deblender:
                 _lib.QuantileReq(fwhm.data_ptr(), 1, good.data_ptr(), 0, n, 0, 0.0)]
         if maxstep_d is not None:
             reqs.append(_lib.QuantileReq(maxstep_d.data_ptr(), 1, None, 1, n, 1, 99 / 100))
-        res = quantiles(reqs)
+        return self._stats_of(quantiles(reqs), maxstep_d is not None)
+
+    @staticmethod
+    def _stats_of(res, steps: bool):
         amplitude = float(res[0, 0]) if res[0, 1] > 0 else 1.0
         width = float(res[1, 0]) if res[1, 1] > 0 else 0.0
-        if maxstep_d is None:
+        if not steps:
             return amplitude, width, np.nan, 0, int(res[0, 1])
         return amplitude, width, float(res[2, 0]), int(res[2, 1]), int(res[0, 1])
 
-    def background_of(self, model, stats):
+    def measure(self, model, params_d, status_d, maxstep_d=None, usable: bool = False):
+        """stats and, unless the background is fixed, the tile medians its next map is made of (of the free
+        pixels and, with ``usable``, of all usable ones), queued together and read back in one download: the
+        thresholds of the free pixels are taken from the stats on the device."""
+        h, w = self.shape
+        tile = self.tile if self.background_level is None else 0
+        ny, nx = (-(-h // tile), -(-w // tile)) if tile else (0, 0)
+        tiles = ny * nx
+        out = dev.empty((6 + (4 if usable else 2) * tiles,), torch.float64)
+        _lib.call("spx_deblend_measure", self.img.data_ptr(), self.dtype, self.sign, h, w, model.data_ptr(),
+                  self.dist2.data_ptr(), _ptr(self.usable_d), params_d.data_ptr(), status_d.data_ptr(), _ptr(maxstep_d),
+                  self.n, float(self.free_fraction), float(self.free_distance_fwhm), tile, int(usable),
+                  out.data_ptr(), self.measure_ws.data_ptr(), self.measure_ws.numel(), dev.stream_ptr())
+        host = dev.start_download(out)
+        torch.cuda.current_stream().synchronize()
+        medians = None
+        if tile:
+            part = host[6:].reshape(-1, ny, nx)
+            medians = (part[0], part[1].view(np.int64), part[2] if usable else None)
+        return self._stats_of(host[:6].reshape(3, 2), maxstep_d is not None), medians
+
+    def background_of(self, model, stats, medians=None):
         """Background map and info (subpx/_cpu/deblend.py:459-466 background_of, 323-393); stats =
-        (median amplitude, median FWHM) of the good cells."""
+        (median amplitude, median FWHM) of the good cells, medians = what `measure` read with them."""
         if self.background_level is not None:
             return self.bg.set_fixed(self.background_level), {"source": "fixed"}
         amplitude, fwhm = stats[0], stats[1]
         tile = self.tile
-        free_med, free_count = self._tile_medians(model, _lib.TILE_FREE, self.free_fraction * amplitude,
-                                                  self.free_distance_fwhm * fwhm)
+        usable_med = None
+        if medians is not None:
+            free_med, free_count, usable_med = medians
+        else:
+            free_med, free_count = self._tile_medians(model, _lib.TILE_FREE, self.free_fraction * amplitude,
+                                                      self.free_distance_fwhm * fwhm)
         measured = free_count >= max(16, int(0.1 * tile * tile))
         info = {"tiles": int(measured.size), "measured_tiles": int(measured.sum())}
         if measured.all():
-            medians, info["source"] = free_med, "measured"
+            medians, info["source"] = np.array(free_med), "measured"  # (free_med may be pinned memory)
         elif measured.any():
             medians, info["source"] = interpolate_tiles(free_med, measured, tile, self.shape), "interpolated"
         else:
-            medians, _ = self._tile_medians(model, _lib.TILE_USABLE)
+            medians = self._tile_medians(model, _lib.TILE_USABLE)[0] if usable_med is None else usable_med
             info["source"] = "inferred"
             if np.isnan(medians).all():
                 whole, _ = self._tile_medians(model, _lib.TILE_ALL, tile=max(self.shape))
@@ -472,21 +501,22 @@ class Deblender:
             init = np.asarray(init, dtype=np.float64)
             params_d = dev.upload(init)
             status_d = self._status_of(params_d)
-        stats = self.stats(params_d, status_d)
         model = self.render(params_d)
+        stats, medians = self.measure(model, params_d, status_d)
         used, converged = 0, False
         for used in range(1, int(iterations) + 1):
-            bg, info = self.background_of(model, stats)
+            bg, info = self.background_of(model, stats, medians)
             params_d, status_d, maxstep_d, it = self.iteration(params_d, model, bg)
             fit_iters.append(it)
             model = self.render(params_d)
-            stats = self.stats(params_d, status_d, maxstep_d)
+            # A page without free tiles rarely gets any: its usable tiles are measured in the same wait.
+            stats, medians = self.measure(model, params_d, status_d, maxstep_d, info["source"] == "inferred")
             if stats[3] == 0:
                 break
             if stats[2] < self.tolerance:
                 converged = True
                 break
-        bg, info = self.background_of(model, stats)
+        bg, info = self.background_of(model, stats, medians)
         self.check_render()
         # Host copies through pinned memory (cached blocks, no fresh pageable arrays to fault in).
         params_h, status_h = dev.start_download(params_d), dev.start_download(status_d)

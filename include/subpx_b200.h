@@ -328,6 +328,17 @@ enum { SPX_TILE_FREE = 0, SPX_TILE_USABLE = 1, SPX_TILE_ALL = 2 };
 int spx_tile_medians(const void* img, int dtype, double sign, int height, int width, const double* model,
                      const unsigned int* dist2, const uint8_t* usable, int mode, double thr_model, double thr_dist,
                      int tile, double* medians, long long* counts, void* stream);
+/* What one pass of the deblending loop reads back, queued without a wait in between: out (device) = the
+ * (value, count) pairs of the median amplitude and the median FWHM of the n >= 1 cells that are ok with A > 0 and
+ * of the 99th percentile of the finite maxstep (null: NaN, 0), then, unless tile is 0, spx_tile_medians' medians
+ * and counts (64-bit integers) of SPX_TILE_FREE with thr_model = free_fraction * amplitude (1 without such cells) and
+ * thr_dist = free_distance_fwhm * FWHM (0), both taken on the device, then with with_usable those of
+ * SPX_TILE_USABLE: 6, 6 + 2 ny nx or 6 + 4 ny nx doubles (subpx/_cpu/deblend.py:459-466, 517). */
+size_t spx_deblend_measure_workspace_bytes(int n);
+int spx_deblend_measure(const void* img, int dtype, double sign, int height, int width, const double* model,
+                        const unsigned int* dist2, const uint8_t* usable, const double* params, const uint8_t* status,
+                        const double* maxstep, int n, double free_fraction, double free_distance_fwhm, int tile,
+                        int with_usable, double* out, void* workspace, size_t workspace_bytes, void* stream);
 /* rows[j][x] = np.interp(x, tile-centre columns, medians[j]) (ny x width). */
 int spx_background_rows(const double* medians, int ny, int nx, int tile, int width, double* rows, void* stream);
 /* Order statistics on the device (np.median / np.percentile 'linear' of a selection), one request
