@@ -56,6 +56,7 @@ int check_launch(const char* what) {
 namespace {
 
 constexpr int kHistSmemBins = 16384;  // value ranges up to this use a shared-memory histogram
+constexpr int kScanPerBlock = 4096;   // bitmap words per prefix block (1024 threads x 4)
 constexpr int kTileH = 32;            // CCL tile (even height keeps 2x2 blocks inside one tile)
 constexpr int kTileW = 64;
 
@@ -64,6 +65,16 @@ constexpr int kTileW = 64;
 __device__ __forceinline__ unsigned int px_u(const void* img, int dtype, long long i) {
     return dtype == SPX_U8 ? (unsigned int)static_cast<const uint8_t*>(img)[i]
                            : (unsigned int)static_cast<const uint16_t*>(img)[i];
+}
+
+// An empty histogram and its range preset, in one launch (a memset and an 8-byte copy from pageable memory cost
+// the host 8 us more).
+__global__ void k_hist_init(unsigned int* hist, int n, unsigned int* range, unsigned int lo, unsigned int hi) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) hist[i] = 0u;
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        range[0] = lo;
+        range[1] = hi;
+    }
 }
 
 // range[0] = min, range[1] = max of the sampled pixels (range must be preset to {~0u, 0}).
@@ -951,6 +962,55 @@ __global__ void k_popc_prefix(const unsigned int* words, long long n, int per_bl
         }
 }
 
+// The three kernels above in one launch, for bitmaps of at most kScanDirect blocks: every block counts the
+// words before its own itself (up to 512 KB from L2) instead of waiting for the others' sums. At 1024 x 1024 4.6
+// instead of 11 us and two launches less; the counting grows with the square of the size: at 2048 x 2048 (32 blocks)
+// 8.4 against 10.7 us for the three kernels at 2100 x 2100.
+constexpr int kScanDirect = 33;
+__global__ void __launch_bounds__(1024) k_popc_prefix_direct(const unsigned int* words, long long n, int* prefix,
+                                                             int* total) {
+    constexpr int kPer = kScanPerBlock / 1024;
+    __shared__ int s_before[32], s_own[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const long long start = (long long)blockIdx.x * kScanPerBlock;
+    int before = 0;
+    const uint4* w4 = reinterpret_cast<const uint4*>(words);
+#pragma unroll 8
+    for (int i = t; i < (int)(start / 4); i += 1024) {
+        const uint4 w = w4[i];
+        before += __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
+    }
+    unsigned w[kPer];
+    int own = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const long long i = start + kPer * t + j;
+        w[j] = i < n ? words[i] : 0u;
+        own += __popc(w[j]);
+    }
+    before = warp_sum_i(before);
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) {
+        s_before[warp] = before;
+        s_own[warp] = incl;
+    }
+    __syncthreads();
+    const int b = warp_sum_i(s_before[lane]), mine = s_own[lane];
+    int run = b + warp_sum_i(lane < warp ? mine : 0) + incl - own;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const long long i = start + kPer * t + j;
+        if (i < n) prefix[i] = run;
+        run += __popc(w[j]);
+    }
+    if (blockIdx.x == gridDim.x - 1 && t == 1023) *total = run;
+}
+
 // --------------------------------------------------------------------------------------- finish
 
 __global__ void k_stats_init(int* stats, unsigned long long* sums, int k1) {
@@ -1197,7 +1257,6 @@ struct CclLayout {
     int* scratch_count;
     unsigned int* fgbits;  // foreground bitmap, H x words-per-row
 };
-constexpr int kScanPerBlock = 4096;  // bitmap words per prefix block (1024 threads x 4)
 
 CclLayout ccl_layout(void* ws, int H, int W, size_t* bytes) {
     CclLayout L;
@@ -1222,17 +1281,6 @@ CclLayout ccl_layout(void* ws, int H, int W, size_t* bytes) {
 // file-scope device array. Every GPU that loads this library holds it (0.25 MiB) until the process exits.
 constexpr size_t kOtsuStaticBytes = 65536 * sizeof(unsigned int) + 2 * 256;
 __device__ __align__(256) unsigned char g_otsu_static[kOtsuStaticBytes];
-
-__global__ void k_range_init(unsigned int* range) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        range[0] = 0xffffffffu;
-        range[1] = 0u;
-    }
-}
-
-__global__ void k_zero_u32(unsigned int* p, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = 0u;
-}
 
 // Device address of g_otsu_static for the current device, looked up once per device and kept for the
 // life of the process: a cudaDeviceReset (which unloads this module's device copy) invalidates it,
@@ -1416,9 +1464,8 @@ int spx_otsu(const void* img, int dtype, int height, int width, int step, double
     unsigned int* hist = a.take<unsigned int>(65536);
     unsigned int* range = a.take<unsigned int>(2);
     const int nbins = dtype == SPX_U8 ? 256 : 65536;
-    SPX_CUDA(cudaMemsetAsync(hist, 0, 65536 * sizeof(unsigned int), s));
-    const unsigned int init[2] = {0xffffffffu, 0u};
-    SPX_CUDA(cudaMemcpyAsync(range, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_hist_init<<<64, 256, 0, s>>>(hist, 65536, range, 0xffffffffu, 0u);
+    if (int e = check_launch("k_hist_init")) return e;
     const int hs = (int)(((long long)height + step - 1) / step), ws = (int)(((long long)width + step - 1) / step);
     const long long n = (long long)hs * ws;
     if (int e = launch_minmax(img, dtype, height, width, step, n, range, s)) return e;
@@ -1438,9 +1485,8 @@ int spx_histogram(const void* img, int dtype, int height, int width, int step, u
     SPX_REQUIRE(height > 0 && width > 0 && step >= 1, "bad image size or step");
     SPX_REQUIRE(img && hist && range, "null pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    SPX_CUDA(cudaMemsetAsync(hist, 0, 65536 * sizeof(unsigned int), s));
-    const unsigned int init[2] = {0xffffffffu, 0u};
-    SPX_CUDA(cudaMemcpyAsync(range, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_hist_init<<<64, 256, 0, s>>>(hist, 65536, range, 0xffffffffu, 0u);
+    if (int e = check_launch("k_hist_init")) return e;
     const int hs = (int)(((long long)height + step - 1) / step), ws = (int)(((long long)width + step - 1) / step);
     const long long n = (long long)hs * ws;
     if (int e = launch_minmax(img, dtype, height, width, step, n, range, s)) return e;
@@ -1481,10 +1527,8 @@ int spx_otsu_static(const void* img, int dtype, int height, int width, int step,
     const int nbins = dtype == SPX_U8 ? 256 : 65536;
     const long long n = hs * ws;
     // The array keeps the previous call's contents: clear the histogram and reset the range first.
-    k_zero_u32<<<64, 256, 0, s>>>(hist, 65536);
-    if (int e = check_launch("k_zero_u32")) return e;
-    k_range_init<<<1, 32, 0, s>>>(range);
-    if (int e = check_launch("k_range_init")) return e;
+    k_hist_init<<<64, 256, 0, s>>>(hist, 65536, range, 0xffffffffu, 0u);
+    if (int e = check_launch("k_hist_init")) return e;
     if (int e = launch_minmax(img, dtype, height, width, step, n, range, s)) return e;
     const size_t smem = kHistSmemBins * sizeof(unsigned int);
     SPX_CUDA(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1506,9 +1550,8 @@ int spx_triangle(const void* img, int dtype, int height, int width, double* thre
     Arena a(workspace);
     unsigned int* hist = a.take<unsigned int>(65536);
     unsigned int* range = a.take<unsigned int>(2);
-    SPX_CUDA(cudaMemsetAsync(hist, 0, 256 * sizeof(unsigned int), s));
-    const unsigned int init[2] = {0u, 255u};
-    SPX_CUDA(cudaMemcpyAsync(range, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_hist_init<<<1, 256, 0, s>>>(hist, 256, range, 0u, 255u);
+    if (int e = check_launch("k_hist_init")) return e;
     const long long n = (long long)height * width;
     const size_t smem = kHistSmemBins * sizeof(unsigned int);
     SPX_CUDA(cudaFuncSetAttribute(k_histogram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1595,6 +1638,10 @@ int spx_ccl_label(const void* img, int dtype, int height, int width, const doubl
     k_border_merge<<<grid_for(border, 256), 256, 0, s>>>(g, L.parents, L.roots, L.fgbits, tiles_x, tiles_y);
     if (int e = check_launch("k_border_merge")) return e;
     SPX_REQUIRE(L.scan_blocks <= 1024 * 64, "image too large for the label prefix");
+    if (L.scan_blocks <= kScanDirect) {
+        k_popc_prefix_direct<<<L.scan_blocks, 1024, 0, s>>>(L.roots, L.words, L.prefix, count);
+        return check_launch("k_popc_prefix_direct");
+    }
     k_popc_block_sums<<<L.scan_blocks, 1024, 0, s>>>(L.roots, L.words, kScanPerBlock, L.block_sums);
     if (int e = check_launch("k_popc_block_sums")) return e;
     k_scan_small<<<1, 1024, 0, s>>>(L.block_sums, L.scan_blocks, count);
