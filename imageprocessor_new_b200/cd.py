@@ -320,6 +320,62 @@ def _start_download(b: dict, after: torch.cuda.Event):
     return h, done
 
 
+# The radial methods' profiles leave the device while later cells are still being measured: cells are taken in
+# chunks of about this many bytes of profile results (at most eight). A page of 116k cells (238 MB) took
+# 75.2 ms with one launch and the download after it, 70.8 ms so; below the size a chunk's copy is shorter than the last,
+# partly filled wave of blocks that every extra launch adds.
+_RADIAL_CHUNK = 32 << 20
+
+
+def _radial_chunks(n: int, row_bytes: int):
+    """[lo, hi) cell ranges of the radial launches."""
+    k = max(1, min(8, n * row_bytes // _RADIAL_CHUNK))
+    edges = [n * i // k for i in range(k + 1)]
+    return list(zip(edges[:-1], edges[1:]))
+
+
+def _offset_out(out: _lib.MethodOut, lo: int, n_angles: int) -> _lib.MethodOut:
+    """The method outputs of the cells from `lo` on."""
+    def at(p, elements, size=8):
+        return None if p is None else p + lo * elements * size
+
+    return _lib.MethodOut(at(out.centers, 2), at(out.contours, 2 * (n_angles + 1)), at(out.status, 1, 1),
+                          at(out.metrics, 1), at(out.center_local, 2), at(out.edge_px, n_angles), None, None,
+                          out.n_metrics, out.metric_col_stride)
+
+
+class _ChunkedDownload:
+    """One method's buffer on its way to pinned host memory: the per-cell rows of its profiles chunk by chunk, the
+    rest at the end. `rows` copies the cells [lo, hi) once the main stream's event has fired."""
+
+    def __init__(self, b: dict):
+        self.flat = b["_flat"]
+        shapes, offsets = b["_layout"]
+        self.host = torch.empty(self.flat.shape, dtype=torch.float64, pin_memory=True)
+        self.parts = [(offsets[k], int(np.prod(shapes[k][1:])), shapes[k][0]) for k in ("contours", "edge_px")
+                      if shapes[k] is not None]
+
+    def rows(self, lo: int, hi: int, after: torch.cuda.Event):
+        side = _copy_stream()
+        side.wait_event(after)
+        with torch.cuda.stream(side):
+            for offset, width, _ in self.parts:
+                part = slice(offset + lo * width, offset + hi * width)
+                self.host[part].copy_(self.flat[part], non_blocking=True)
+
+    def finish(self, after: torch.cuda.Event):
+        side = _copy_stream()
+        side.wait_event(after)
+        with torch.cuda.stream(side):
+            at = 0
+            for offset, width, count in sorted(self.parts) + [(self.flat.numel(), 0, 0)]:
+                self.host[at:offset].copy_(self.flat[at:offset], non_blocking=True)
+                at = offset + width * count
+            done = torch.cuda.Event()
+            done.record(side)
+        return self.host, done
+
+
 def _to_result(method: str, n: int, b: dict, host: np.ndarray, metrics_only: bool, n_angles: int) -> CDMethodResult:
     names = _metric_names(method)
     shapes, offsets = b["_layout"]
@@ -563,7 +619,7 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
     bufs, pending = {}, []  # pending: (method names, host copies and their completion events)
     main = torch.cuda.current_stream()
 
-    def launched(names):
+    def launched(names, copies=None):
         # Each method's results go to pinned host memory on a side stream as soon as its kernel is
         # done, so the host converts one method while the GPU still runs the next.
         for name in names:
@@ -571,7 +627,10 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
             _lib.call("spx_status_text", b["status"].data_ptr(), nr, b["status_text"].data_ptr(), stream)
         ev = torch.cuda.Event()
         ev.record(main)
-        pending.append((names, [_start_download(bufs[name], ev) for name in names]))
+        if copies is not None:
+            pending.append((names, [copy.finish(ev) for copy in copies]))
+        else:
+            pending.append((names, [_start_download(bufs[name], ev) for name in names]))
 
     t_gauss = time.perf_counter()
     if "gaussian" in methods and nr:
@@ -598,15 +657,29 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
             weights, smooth_r = gaussian_weights(smooth_sigma)
             smooth_w = dev.upload(weights)
         ws = dev.workspace(_lib.size("spx_radial_workspace_bytes", c.hm, c.wm, int(smooth_w is not None)))
-        _lib.call("spx_radial_cd", cleaned.data_ptr(), c.voronoi.data_ptr(), c.boxes.data_ptr(), report_d.data_ptr(),
-                  nr, c.hm, c.wm, width, n_angles, radial_step, dev.ptr(smooth_w), smooth_r,
-                  None if hb[1] is None else hb[1], None if gb[1] is None else gb[1], ws.data_ptr(), ws.numel(),
-                  stream)
         if hb[0] is not None:
             bufs["halfmax"] = hb[0]
         if gb[0] is not None:
             bufs["gradient"] = gb[0]
-        launched([m for m in ("halfmax", "gradient") if m in bufs])
+        names = [m for m in ("halfmax", "gradient") if m in bufs]
+        copies = None
+        row_bytes = len(names) * 8 * (n_angles if metrics_only else 3 * n_angles + 2)
+        chunks = _radial_chunks(nr, row_bytes)
+        if len(chunks) > 1:
+            copies = [_ChunkedDownload(bufs[m]) for m in names]
+        for lo, hi in chunks:
+            _lib.call("spx_radial_cd", cleaned.data_ptr() + lo * c.hm * c.wm * 8, c.voronoi.data_ptr(),
+                      c.boxes.data_ptr(), report_d.data_ptr() + lo * 4, hi - lo, c.hm, c.wm, width, n_angles,
+                      radial_step, dev.ptr(smooth_w), smooth_r,
+                      None if hb[1] is None else _offset_out(hb[1], lo, n_angles),
+                      None if gb[1] is None else _offset_out(gb[1], lo, n_angles), ws.data_ptr(), ws.numel(),
+                      stream)
+            if copies is not None:
+                ev = torch.cuda.Event()
+                ev.record(main)
+                for copy in copies:
+                    copy.rows(lo, hi, ev)
+        launched(names, copies)
     seconds["radial"] = time.perf_counter() - start - t_gauss
     t_proj = time.perf_counter()
     if "projection" in methods and nr:
