@@ -247,6 +247,12 @@ def measure_cds(
 
 
 def _segment(img_d: torch.Tensor, threshold: str, invert: bool):
+    """The components of `_segment_start`, counted, and whether the image was rescaled."""
+    started, rescaled = _segment_start(img_d, threshold, invert)
+    return segment.label_finish(started, dev.read_int(started.count)), rescaled
+
+
+def _segment_start(img_d: torch.Tensor, threshold: str, invert: bool, count: torch.Tensor | None = None):
     """Binary components of the reference's segmentation (subpx/cd.py:472-481): uint8 and uint16 +
     Otsu images are thresholded as they are, others are scaled to uint8 first."""
     rescaled = img_d.dtype != torch.uint8 and not (img_d.dtype == torch.uint16 and threshold == "otsu")
@@ -260,8 +266,7 @@ def _segment(img_d: torch.Tensor, threshold: str, invert: bool):
         else:
             seg = torch.zeros(img_d.shape, dtype=torch.uint8, device="cuda")
     thr = segment.binarize_threshold(seg, threshold, invert)
-    comp = segment.label(seg, threshold=thr, invert=invert, connectivity=8)
-    return comp, rescaled
+    return segment.label_start(seg, threshold=thr, invert=invert, connectivity=8, count=count), rescaled
 
 
 def _method_buffers(n: int, n_angles: int, method: str, contours: bool):

@@ -58,6 +58,13 @@ def build_cells(rows, shape, pad: int, rows_d: torch.Tensor | None = None) -> Ce
 
     With ``rows_d`` (the rows already on the device) ``rows`` may be a host array whose copy from
     the device is still in flight on the current stream: it is read only after the stream syncs."""
+    finish = build_cells_start(rows, shape, pad, rows_d)
+    torch.cuda.current_stream().synchronize()
+    return finish()
+
+
+def build_cells_start(rows, shape, pad: int, rows_d: torch.Tensor | None = None):
+    """build_cells without its wait: the function it returns gives the Cells once the stream has synced."""
     h, w = shape
     if rows_d is None:
         rows = np.asarray(rows, dtype=np.float64).reshape(-1, 6)
@@ -74,15 +81,18 @@ def build_cells(rows, shape, pad: int, rows_d: torch.Tensor | None = None) -> Ce
               counts.data_ptr(), caps.data_ptr(), dev.stream_ptr())
     host = dev.start_download(boxes[:n])
     host_counts = dev.start_download(counts[:n])
-    torch.cuda.current_stream().synchronize()
-    rows = np.asarray(rows, dtype=np.float64).reshape(-1, 6)
-    hm = int(host[:, 3].max()) if n else 0
-    wm = int(host[:, 2].max()) if n else 0
-    max_px = int(host_counts.max()) if n else 1
-    # Seeds, origins and sizes are views of the downloaded arrays (new host arrays of this size
-    # cost more in first-touch page faults than the copies themselves).
-    return Cells(rows, rows[:, 4:6], seeds_d, vor, boxes[:n], counts[:n], caps[:n], host[:, :2], host[:, 2:4], hm,
-                 wm, max(max_px, 1))
+
+    def finish() -> Cells:
+        host_rows = np.asarray(rows, dtype=np.float64).reshape(-1, 6)
+        hm = int(host[:, 3].max()) if n else 0
+        wm = int(host[:, 2].max()) if n else 0
+        max_px = int(host_counts.max()) if n else 1
+        # Seeds, origins and sizes are views of the downloaded arrays (new host arrays of this size
+        # cost more in first-touch page faults than the copies themselves).
+        return Cells(host_rows, host_rows[:, 4:6], seeds_d, vor, boxes[:n], counts[:n], caps[:n], host[:, :2],
+                     host[:, 2:4], hm, wm, max(max_px, 1))
+
+    return finish
 
 
 def auto_tile(seeds_d: torch.Tensor, n: int, shape) -> tuple[int, float]:

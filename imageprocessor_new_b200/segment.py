@@ -52,25 +52,48 @@ def triangle(img: torch.Tensor) -> torch.Tensor:
     return out
 
 
+@dataclass
+class Labelled:
+    """Components found but not yet counted on the host: label_start's work, label_finish's input."""
+
+    labels: torch.Tensor
+    count: torch.Tensor  # one device int
+    workspace: torch.Tensor
+    connectivity: int
+
+
+def label_start(img: torch.Tensor, *, threshold: torch.Tensor | None = None, fixed_threshold: float = 0.0,
+                invert: bool = False, connectivity: int = 8, count: torch.Tensor | None = None) -> Labelled:
+    """The part of `label` before its component count is known (nothing synchronises); ``count`` receives it."""
+    h, w = img.shape
+    code = dev.dtype_code(img)
+    labels = dev.empty((h, w), torch.int32)
+    count = dev.empty((1,), torch.int32) if count is None else count
+    ws = dev.workspace(_lib.size("spx_ccl_workspace_bytes", h, w))
+    _lib.call("spx_ccl_label", img.data_ptr(), code, h, w, dev.ptr(threshold), float(fixed_threshold),
+              int(bool(invert)), int(connectivity), labels.data_ptr(), count.data_ptr(), ws.data_ptr(),
+              ws.numel(), dev.stream_ptr())
+    return Labelled(labels, count, ws, int(connectivity))
+
+
+def label_finish(started: Labelled, k: int) -> Components:
+    """Labels, stats and centroids of the ``k`` components label_start counted."""
+    h, w = started.labels.shape
+    stats = dev.empty((k + 1, 5), torch.int32)
+    centroids = dev.empty((k + 1, 2), torch.float64)
+    ws = started.workspace
+    _lib.call("spx_ccl_finish", started.labels.data_ptr(), h, w, started.connectivity, k, stats.data_ptr(),
+              centroids.data_ptr(), ws.data_ptr(), ws.numel(), dev.stream_ptr())
+    return Components(started.labels, stats, centroids, k)
+
+
 def label(img: torch.Tensor, *, threshold: torch.Tensor | None = None, fixed_threshold: float = 0.0,
           invert: bool = False, connectivity: int = 8) -> Components:
     """Binarise (img > t, or img <= t with invert) and label 8/4-connected components, numbered as
     cv2.connectedComponentsWithStats numbers them, with their stats and centroids."""
-    h, w = img.shape
-    code = dev.dtype_code(img)
-    labels = dev.empty((h, w), torch.int32)
-    count = dev.empty((1,), torch.int32)
-    ws = dev.workspace(_lib.size("spx_ccl_workspace_bytes", h, w))
-    stream = dev.stream_ptr()
-    _lib.call("spx_ccl_label", img.data_ptr(), code, h, w, dev.ptr(threshold), float(fixed_threshold),
-              int(bool(invert)), int(connectivity), labels.data_ptr(), count.data_ptr(), ws.data_ptr(),
-              ws.numel(), stream)
-    k = dev.read_int(count)
-    stats = dev.empty((k + 1, 5), torch.int32)
-    centroids = dev.empty((k + 1, 2), torch.float64)
-    _lib.call("spx_ccl_finish", labels.data_ptr(), h, w, int(connectivity), k, stats.data_ptr(),
-              centroids.data_ptr(), ws.data_ptr(), ws.numel(), stream)
-    return Components(labels, stats, centroids, k)
+    started = label_start(img, threshold=threshold, fixed_threshold=fixed_threshold, invert=invert,
+                          connectivity=connectivity)
+    return label_finish(started, dev.read_int(started.count))
 
 
 def binarize_threshold(img: torch.Tensor, threshold: str, invert: bool) -> torch.Tensor:
