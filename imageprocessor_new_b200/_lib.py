@@ -109,6 +109,7 @@ SIGNATURES = {
     "spx_morphology": (_I, [_P, _I, _I, _I, _I, _P, _P]),
     "spx_ccl_label": (_I, [_P, _I, _I, _I, _P, _D, _I, _I, _P, _P, _P, _S, _P]),
     "spx_ccl_finish": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _S, _P]),
+    "spx_ccl_finish_counted": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _P, _S, _P]),
     "spx_select_workspace_bytes": (_S, [_I]),
     "spx_select_components": (_I, [_P, _I, _I, _I, _I, _D, _P, _P, _P, _P, _S, _P]),
     "spx_component_rows": (_I, [_P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _S, _P]),

@@ -80,11 +80,13 @@ def _segmentation_source(img_d: torch.Tensor, threshold_dev, fixed_threshold: fl
 def _centers_on_device(img_d: torch.Tensor, *, threshold_dev: torch.Tensor | None, fixed_threshold: float,
                        invert: bool, area_min: int, area_max: int, pad: int, refine: str,
                        connectivity: int, small_feature_max: float, morph_open: int = 0,
-                       morph_close: int = 0) -> torch.Tensor:
-    """Refined centres (n, 2) on the device, NaN rows for failed refinements, in label order."""
-    src, thr, fixed, inv = _segmentation_source(img_d, threshold_dev, fixed_threshold, invert, morph_open,
-                                                morph_close)
-    comp = segment.label(src, threshold=thr, fixed_threshold=fixed, invert=inv, connectivity=connectivity)
+                       morph_close: int = 0, comp: segment.Components | None = None) -> torch.Tensor:
+    """Refined centres (n, 2) on the device, NaN rows for failed refinements, in label order; ``comp``: the
+    image's components, when they are labelled already."""
+    if comp is None:
+        src, thr, fixed, inv = _segmentation_source(img_d, threshold_dev, fixed_threshold, invert, morph_open,
+                                                    morph_close)
+        comp = segment.label(src, threshold=thr, fixed_threshold=fixed, invert=inv, connectivity=connectivity)
     k = comp.count
     h, w = img_d.shape
     rows = dev.empty((max(k, 1), 5), torch.int32)
@@ -102,38 +104,42 @@ def _centers_on_device(img_d: torch.Tensor, *, threshold_dev: torch.Tensor | Non
     return centers[:n]
 
 
-# Frames of up to this many pixels are measured with room for a component in every 64 of them: the device keeps
-# the counts and the host waits once, for the result, instead of also for the component count and the kept count.
-# Threshold to result, one wait against three: 512 x 512 177 and 210, 1024 x 1024 194 and 219, 1448 x 1448 225 and
-# 245, 2048 x 2048 256 and 263, 2100 x 2100 272 and 272 us (the empty rows' share grows).
+# Frames of up to this many pixels are measured with room for a component in every 16 of them (random pixels
+# leave one in about 20 at the densest), beyond 16,384 rows for one in every 64: the device keeps the counts and the
+# host waits once, for the result, instead of also for the component count and the kept count. Threshold to result,
+# one wait against three: 512 x 512 190 and 213, 1024 x 1024 202 and 217, 1448 x 1448 231 and 244, 2048 x 2048 264 and
+# 278 us (the empty rows' share grows, and so does what a frame with too many components spends in vain). Frames
+# of random pixels: 512 x 512 259 instead of 327 us with room for one in 64, 1024 x 1024 (too many) 420-440 either way.
 _ONE_WAIT_PIXELS = 1 << 21
 
 
 def _centers_in_one_wait(img_d: torch.Tensor, *, threshold_dev: torch.Tensor | None, fixed_threshold: float,
                          invert: bool, area_min: int, area_max: int, pad: int, refine: str, connectivity: int,
-                         small_feature_max: float, morph_open: int = 0, morph_close: int = 0) -> np.ndarray | None:
+                         small_feature_max: float, morph_open: int = 0, morph_close: int = 0,
+                         overflow: list | None = None) -> np.ndarray | None:
     """_finite(_centers_on_device(...)) with one wait; None when the frame has more components than there is
-    room for."""
+    room for: the device then leaves the tables empty, and the labelling, finished with its true count, is
+    appended to ``overflow``."""
     src, thr, fixed, inv = _segmentation_source(img_d, threshold_dev, fixed_threshold, invert, morph_open,
                                                 morph_close)
     h, w = img_d.shape
     stream = dev.stream_ptr()
-    cap = max(h * w // 64, 64)
-    labels = dev.empty((h, w), torch.int32)
+    cap = max(min(h * w // 16, max(16384, h * w // 64)), 64)
     # centres, then component and kept counts: what comes back, in one copy
     out = dev.empty((2 * cap + 1,), torch.float64)
-    counts = out.data_ptr() + 16 * cap
+    count = out[2 * cap:].view(torch.int32)
+    counts = count.data_ptr()
     # (the component statistics' 64-bit sums live in the centroid array)
     table = dev.empty((cap + 1, 2), torch.float64)
     rows = dev.empty((2, cap + 1, 5), torch.int32)
     methods = dev.empty((cap,), torch.uint8)
-    ws = dev.workspace(_lib.size("spx_ccl_workspace_bytes", h, w))
     sel_ws = dev.workspace(_lib.size("spx_select_workspace_bytes", cap))
     code = _lib.REFINE_CODES[refine]
-    _lib.call("spx_ccl_label", src.data_ptr(), dev.dtype_code(src), h, w, dev.ptr(thr), float(fixed), int(bool(inv)),
-              int(connectivity), labels.data_ptr(), counts, ws.data_ptr(), ws.numel(), stream)
-    _lib.call("spx_ccl_finish", labels.data_ptr(), h, w, int(connectivity), cap, rows[0].data_ptr(), table.data_ptr(),
-              ws.data_ptr(), ws.numel(), stream)
+    started = segment.label_start(src, threshold=thr, fixed_threshold=fixed, invert=inv, connectivity=connectivity,
+                                  count=count)
+    labels, ws = started.labels, started.workspace
+    _lib.call("spx_ccl_finish_counted", labels.data_ptr(), h, w, int(connectivity), cap, counts, rows[0].data_ptr(),
+              table.data_ptr(), ws.data_ptr(), ws.numel(), stream)
     _lib.call("spx_select_components", rows[0].data_ptr(), cap, int(area_min), int(area_max), code,
               float(small_feature_max), rows[1].data_ptr(), methods.data_ptr(), counts + 4, sel_ws.data_ptr(),
               sel_ws.numel(), stream)
@@ -143,6 +149,8 @@ def _centers_in_one_wait(img_d: torch.Tensor, *, threshold_dev: torch.Tensor | N
     torch.cuda.current_stream().synchronize()
     found, kept = host[2 * cap:].view(np.int32)
     if found > cap:
+        if overflow is not None:
+            overflow.append(segment.label_finish(started, int(found)))
         return None
     return _finite_rows(np.array(host[:2 * kept]).reshape(-1, 2))
 
@@ -237,9 +245,10 @@ def detect_centers(
                       morph_open=int(morph_open), morph_close=int(morph_close))
         # (An area_min below 1 would take the table's empty rows for components.)
         small = img_d.numel() <= _ONE_WAIT_PIXELS and area_min >= 1
-        arr = _centers_in_one_wait(img_d, **common) if small else None
+        overflow = []
+        arr = _centers_in_one_wait(img_d, overflow=overflow, **common) if small else None
         if arr is None:
-            arr = _finite(_centers_on_device(img_d, **common))
+            arr = _finite(_centers_on_device(img_d, comp=overflow[0] if overflow else None, **common))
     meta = {
         "invert": bool(invert), "area_min": int(area_min), "area_max": int(area_max),
         "morph_open": int(morph_open), "morph_close": int(morph_close), "pad": int(pad),

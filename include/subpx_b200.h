@@ -149,6 +149,10 @@ int spx_ccl_label(const void* img, int dtype, int height, int width, const doubl
 int spx_ccl_finish(int* labels, int height, int width, int connectivity, int num_components,
                    int* stats, double* centroids, void* workspace, size_t workspace_bytes,
                    void* stream);
+/* spx_ccl_finish with tables for `capacity` components while the true number is still in *count (device):
+ * rows past the count stay empty (area 0); with more components than rows no label and no row is written. */
+int spx_ccl_finish_counted(int* labels, int height, int width, int connectivity, int capacity, const int* count,
+                           int* stats, double* centroids, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Component selection and centre refinement.
