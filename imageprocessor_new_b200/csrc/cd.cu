@@ -1111,8 +1111,10 @@ __device__ __forceinline__ void ray_edges64(const double* coef, int hp, int wp, 
 // Bound: instructions (about 100,000 a cell of 24 px pitch, 128 rays of 110 samples: half of them the walk's,
 // a quarter the spline coefficients and masks, the rest the FP64 edges). With FP64 positions the walk spent 47
 // FP64 instructions a sample and 32 separate exits a warp; FP32 positions with one cheap exit test, box indices
-// without integer divisions: 29,000 such cells 4.67 -> 4.17 ms. Five blocks per SM without spills measure the
-// same (4.15), the sample taken before the validity test 4.30, the loop unrolled by two 4.60.
+// without integer divisions: 29,000 such cells 4.67 -> 3.99 ms (4.17 with the position's bound taken from the longest
+// radius instead of the box's reach: more rays walked again); pitches of 14 to 60 px 12-14 % less each. Against 4.17:
+// five blocks per SM without spills measure the same (4.15), the sample taken before the validity test 4.30, the loop
+// unrolled by two 4.60.
 template <bool kSmooth, int kRays>
 __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
     const double* cleaned, const int* vor, const int4* boxes, const int* which, int n, int hm, int wm, int W,
@@ -1250,13 +1252,14 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
             quad[k] = f;
             cmax = fmaxf(cmax, fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
         }
-        // A sample's FP32 position is within perr = (4 R + 2) 2^-24 pixels of the FP64 one (R the longest radius:
-        // the roundings of step, radius, direction, sum and centre). The window weights are non-negative and sum
-        // to one per axis, their derivatives' magnitudes to at most 1.5, so a sample is within about 45 ulps of
-        // cmax (coefficient and weight roundings, 20 FMAs) + 3 perr cmax of the FP64 one; tol keeps a margin
-        // (2^-17 cmax + 4 perr cmax). Also orders the quad writes before the rays read them.
+        // A sample's FP32 position is within perr = (4 X + 2) 2^-24 pixels of the FP64 one in each axis (X: the box's
+        // farthest side from the centre, plus one; the roundings of step, radius, direction, sum and centre). The
+        // window weights are non-negative and sum to one per axis, their derivatives' magnitudes to at most 1.5, so a
+        // sample is within about 45 ulps of cmax (coefficient and weight roundings, 20 FMAs) + 3 perr cmax of the FP64
+        // one; tol keeps a margin (2^-17 cmax + 4 perr cmax). Also orders the quad writes before the rays read them.
         if (tid == 0) s_nq = 0;  // before the barrier in cta_max; read after the barrier that follows the rays
-        const float perr = (4.0f * (float)(n_radii * radial_step) + 2.0f) * 5.9604644775390625e-08f;
+        const double reach = fmax(fmax(cx, (double)(wm - 1) - cx), fmax(cy, (double)(hm - 1) - cy)) + 1.0;
+        const float perr = (4.0f * (float)reach + 2.0f) * 5.9604644775390625e-08f;
         const float tol = (float)cta_max((double)cmax, red + 28) * 36.0f * (7.62939453125e-06f + 4.0f * perr);
         const float inner = 0.5f - 2.0f * perr;
         const float stepf = (float)radial_step;

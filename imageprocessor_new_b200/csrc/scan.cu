@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_one_block(const int* in, 
             v[i] = next[i];
             acc += v[i];
         }
-        load(base + kScanTile);  // (in place: items past this round are not written yet)
+        load(base + kScanTile);  // (in place: items past this step are not written yet)
         int incl = acc;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
