@@ -9,9 +9,11 @@
 // Cells are implicit: cell j is box j (origin, size) intersected with Voronoi label j, so no mask
 // stack is stored. A fit kernel stages each cell's cleaned pixels (image - background - (model -
 // own model)) once into the warp's shared-memory slice and runs the whole LM loop there; a work
-// queue hands cells to persistent warps. The model image is gathered, not scattered: each 16x16
-// tile sums the truncated Gaussians that reach it in increasing cell order (NumPy's bincount order),
+// queue hands cells to persistent warps. The model image is gathered, not scattered: each tile
+// of pixels sums the truncated Gaussians that reach it in increasing cell order (NumPy's bincount order),
 // so it is deterministic without atomics.
+
+#include <type_traits>
 
 #include "bins.cuh"
 #include "image.cuh"
@@ -539,7 +541,8 @@ __global__ void k_render_prep(const double* params, const int4* boxes, int n, in
 // Render tiles: kRenderTile x kRenderTile pixels per block (16, 32 or 64 px; larger tiles gather their
 // candidates less often).
 constexpr int kRenderCap = 2048;
-constexpr int kRenderThreads = 128;
+// Threads of a block: its warps own whole columns of patches, and 64 px have eight.
+constexpr int render_threads(int tile) { return tile == 64 ? 256 : 128; }
 
 // model(y, x) = sum over cells (increasing index) whose truncated square covers the pixel, each
 // term A exp(-(a^2 + b^2) / 2) for |x - X0| <= r and |y - Y0| <= r (render_models).
@@ -548,11 +551,12 @@ constexpr int kRenderThreads = 128;
 // column of 8 x 4 px patches, so a 37 px square that cuts a patch leaves few of its lanes idle (78 % busy;
 // 32 x 1 px rows: 52 %), and skips candidates that miss its columns with one test. Measured on the 8192 page
 // (116k Gaussians): 64 px tiles, 256 threads, rows of 32: 0.97 ms; patches 0.93 ms; 32 px tiles 0.80 ms, with
-// 128 threads 0.73 ms.
+// 128 threads 0.73 ms. With binning, on a lattice of that size: 16, 32 and 64 px tiles 1.08, 0.77 and 0.97 ms.
 template <int kRenderTile>
-__global__ void __launch_bounds__(kRenderThreads) k_render(int H, int W, BinGrid g, const double* params,
+__global__ void __launch_bounds__(render_threads(kRenderTile)) k_render(int H, int W, BinGrid g, const double* params,
                                                const double* centres, const int* radius,
                                                const int* rmax_dev, double* model, int* overflow) {
+    constexpr int kRenderThreads = render_threads(kRenderTile), kWarps = kRenderThreads / 32;
     __shared__ int cand[kRenderCap];
     __shared__ int s_n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(kRenderThreads) k_render(int H, int W, BinGrid
     const int gy0 = bin_index((double)(ty0 - rmax - 1), g.cell, g.gh);
     const int gy1 = bin_index((double)(ty1 + rmax + 1), g.cell, g.gh);
     // One warp per bin row, so that the rows' chains of loads (offsets, points, radii) run side by side.
-    for (int gy = gy0 + warp; gy <= gy1; gy += kRenderThreads / 32) {
+    for (int gy = gy0 + warp; gy <= gy1; gy += kWarps) {
         const int j0 = g.start[gy * g.gw + gx0], j1 = g.start[gy * g.gw + gx1 + 1];
         for (int k = j0 + lane; k < j1; k += 32) {
             const int id = g.id[k];
@@ -602,7 +606,8 @@ __global__ void __launch_bounds__(kRenderThreads) k_render(int H, int W, BinGrid
     __shared__ double s_e1[kRenderThreads], s_u2[kRenderThreads], s_e3[kRenderThreads];
     __shared__ int4 s_box[kRenderThreads];  // x lo, x hi, y lo, y hi
     constexpr int kCols = kRenderTile / 8;                 // patch columns
-    constexpr int kRows = (kRenderTile / 4) * kCols / (kRenderThreads / 32);   // patches of a warp, one below the other
+    constexpr int kRows = (kRenderTile / 4) * kCols / kWarps;  // patches of a warp, one below the other
+    static_assert(kWarps % kCols == 0 && 4 * kRows * (kWarps / kCols) == kRenderTile, "the patches cover the tile once");
     const int px0 = tx0 + 8 * (warp % kCols), py0 = ty0 + 4 * kRows * (warp / kCols);
     const int x = px0 + (lane & 7), yb = py0 + (lane >> 3);
     double acc[kRows];
@@ -1399,15 +1404,14 @@ int spx_render_model(const double* params, const int* boxes, int n, int height, 
     auto tiles = [&](int t) { return (long long)((width + t - 1) / t) * ((height + t - 1) / t); };
     while (tile > 16 && tiles(tile) < 4 * 148) tile /= 2;
     const dim3 grid((width + tile - 1) / tile, (height + tile - 1) / tile);
-    if (tile == 16)
-        k_render<16><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
-                                          L.overflow);
-    else if (tile == 64)
-        k_render<64><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
-                                          L.overflow);
-    else
-        k_render<32><<<grid, kRenderThreads, 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius, L.rmax, model,
-                                          L.overflow);
+    auto render = [&](auto edge) {
+        constexpr int kTile = decltype(edge)::value;
+        k_render<kTile><<<grid, render_threads(kTile), 0, s>>>(height, width, bin_view(L.bins), params, L.centres, L.radius,
+                                                               L.rmax, model, L.overflow);
+    };
+    if (tile == 16) render(std::integral_constant<int, 16>{});
+    else if (tile == 64) render(std::integral_constant<int, 64>{});
+    else render(std::integral_constant<int, 32>{});
     return check_launch("k_render");
 }
 
