@@ -12,7 +12,9 @@ the keep rule drops), and the host reads the per-band component counts once at t
 capacity is twice the components of the band the graph was built on; a page with a band of more
 components than that is redone by the eager path (and the graph rebuilt, for that many, on the next
 call). Idle graphs wait in a small pool; a call takes the ones it uses out of it and puts them back
-once its work has finished, so calls from several threads or on several streams never share one."""
+once its work has finished, so calls from several threads or on several streams never share one. A
+graph is captured by a call that runs alone: one that overlaps another and finds no idle graph takes
+the eager path, and the capture leaves other threads free to allocate and copy."""
 
 from __future__ import annotations
 
@@ -98,9 +100,16 @@ class BandGraph:
                         float(small_feature_max))
         self.graph = torch.cuda.CUDAGraph()
         self._launch()  # eager once: first launches and attribute settings happen outside the capture
-        torch.cuda.synchronize()
-        with torch.cuda.graph(self.graph):
-            self._launch()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            # Thread-local: the default mode refuses other threads' allocations while a capture is under way, and an
+            # allocation that is refused ends the capture too.
+            self.graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                self._launch()
+            finally:
+                self.graph.capture_end()
 
     def _launch(self):
         h, w = self.shape
@@ -133,6 +142,7 @@ class BandGraph:
 _GRAPHS: dict = {}      # key -> idle graphs of that key
 _COMPONENTS: dict = {}  # key -> components of the fullest band that overflowed a graph of that key
 _GRAPHS_MOST = 4        # idle graphs kept
+_CALLS = 0              # calls that hold or capture graphs
 _GRAPHS_LOCK = threading.Lock()
 
 
@@ -140,6 +150,23 @@ def _take_graph(key):
     with _GRAPHS_LOCK:
         idle = _GRAPHS.get(key)
         return idle.pop() if idle else None
+
+
+def _begin_call(keys):
+    """The graphs a call may go by, {key: an idle one, or None: to be captured}; None when one is missing while
+    another call runs. Ended with _end_call."""
+    global _CALLS
+    with _GRAPHS_LOCK:
+        if _CALLS and not all(_GRAPHS.get(k) for k in keys):
+            return None
+        _CALLS += 1
+        return {k: _GRAPHS[k].pop() if _GRAPHS.get(k) else None for k in keys}
+
+
+def _end_call():
+    global _CALLS
+    with _GRAPHS_LOCK:
+        _CALLS -= 1
 
 
 def _put_graph(key, graph):
@@ -163,15 +190,26 @@ def _keep_bands(bands, kept_rows):
 
 def _bands_with_graphs(img_d, spans, thr, common):
     """Every band through a BandGraph of its height at the device threshold; None when a band overflows
-    its capacity."""
+    its capacity, or when a graph would have to be captured while another call runs."""
+    keys = {y1 - y0: (y1 - y0, img_d.shape[1], img_d.dtype, tuple(sorted(common.items())), torch.cuda.current_device(),
+                      BAND_PX_PER_COMPONENT) for y0, y1, _, _ in spans}
+    idle = _begin_call(list(keys.values()))
+    if idle is None:
+        return None
+    try:
+        return _run_graphs(img_d, spans, thr, common, keys, idle)
+    finally:
+        _end_call()
+
+
+def _run_graphs(img_d, spans, thr, common, keys, idle):
     width = img_d.shape[1]
     graphs = {}  # band height -> (key, graph), this call's own until they are put back
     for y0, y1, _, _ in spans:
         if y1 - y0 in graphs:
             continue
-        key = (y1 - y0, width, img_d.dtype, tuple(sorted(common.items())), torch.cuda.current_device(),
-               BAND_PX_PER_COMPONENT)
-        graph = _take_graph(key)
+        key = keys[y1 - y0]
+        graph = idle[key]
         if graph is None:
             graph = BandGraph(y1 - y0, width, img_d.dtype, threshold=thr, sample=img_d[y0:y1],
                               components=_COMPONENTS.get(key, 0), **common)

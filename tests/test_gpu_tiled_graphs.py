@@ -86,3 +86,64 @@ def test_calls_from_several_threads_do_not_share_a_graph():
     with ThreadPoolExecutor(1) as pool:  # another thread and stream than the graphs were built on
         for k, got in enumerate(pool.map(run, range(4))):
             np.testing.assert_array_equal(got, want[k])
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_a_capture_leaves_overlapping_calls_alone(monkeypatch, warm):
+    """While one thread captures its first graph another allocates device and pinned memory and runs whole calls, from
+    an empty pool and with idle graphs of its own: both succeed with the eager path's centres."""
+    import threading
+
+    import torch
+
+    from imageprocessor_new_b200 import detect_centers, tiled
+
+    first, second = _page(20), _page(21, holes=0.6)[:, :380]
+    want = [_eager(first), _eager(second)]
+    tiled._GRAPHS.clear()
+    if warm:
+        detect_centers(second, backend="gpu", **KW)
+    capturing, other_done, failed, got = threading.Event(), threading.Event(), [], {}
+    launch = tiled.BandGraph._launch
+
+    def slow_launch(self):
+        if self.shape[1] == first.shape[1] and torch.cuda.is_current_stream_capturing() and not capturing.is_set():
+            capturing.set()
+            assert other_done.wait(60)
+        launch(self)
+
+    monkeypatch.setattr(tiled.BandGraph, "_launch", slow_launch)
+
+    def capture():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got["first"] = detect_centers(first, backend="gpu", **KW)
+
+    def others():
+        try:
+            assert capturing.wait(60)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                held = [torch.empty(96 << 20, dtype=torch.uint8, device="cuda"),
+                        torch.empty(48 << 20, dtype=torch.uint8, pin_memory=True)]
+                for _ in range(3):
+                    got["second"] = detect_centers(second, backend="gpu", **KW)
+                del held
+        finally:
+            other_done.set()
+
+    def run(fn):
+        try:
+            fn()
+        except BaseException as e:
+            failed.append(e)
+
+    threads = [threading.Thread(target=run, args=(f,)) for f in (capture, others)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    assert capturing.is_set()
+    np.testing.assert_array_equal(got["first"].centers_xy, want[0])
+    np.testing.assert_array_equal(got["second"].centers_xy, want[1])
+    assert got["first"].meta["band_graphs"] and got["second"].meta["band_graphs"] == warm
+    tiled._GRAPHS.clear()
