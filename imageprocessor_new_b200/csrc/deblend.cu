@@ -654,15 +654,24 @@ __global__ void __launch_bounds__(render_threads(kRenderTile)) k_render(int H, i
         }
 }
 
+constexpr int kChipWarps = 148 * 64;  // warps the chip holds at a time
+
 // Cleaned cells (image - background - (model - own)) of the cells in `which` (all when null) as
 // an (n_out, hm, wm) stack, zero outside each cell (DeblendState.cleaned). One warp per cell: the widths and the
 // radius of its Gaussian are computed once a lane instead of once a pixel (29k cells of 24 px
-// pitch 0.263 -> 0.179 ms; the fused multiply-adds are the per-pixel form's).
+// pitch 0.263 -> 0.179 ms; the fused multiply-adds are the per-pixel form's). Fewer cells than the chip holds
+// warps are cut into `parts` of every parts-th 32 pixels, a warp each. us with a thread per pixel / a warp per cell /
+// parts: one 200 px cell 12.7 / 978 / 7.9, ten of 500 px 44 / 7280 / 24, 1,000 of 30 px 19 / 29 / 15, 6,000 of
+// 24 px 68 / 42 / 42.
 __global__ void __launch_bounds__(256) k_clean_stack(Image img, const int* vor, const int4* boxes, const double* params,
                                                      int radius_cap, spx_bgmap bg, const double* model,
-                                                     const int* which, int n_out, int hm, int wm, double* out) {
+                                                     const int* which, int n_out, int parts, int hm, int wm,
+                                                     double* out) {
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, area = hm * wm;
-    for (int c = blockIdx.x * warps + (threadIdx.x >> 5); c < n_out; c += gridDim.x * warps) {
+    const long long units = (long long)n_out * parts;
+    for (long long u = blockIdx.x * (long long)warps + (threadIdx.x >> 5); u < units; u += (long long)gridDim.x * warps) {
+        int c, part;
+        divmod_idx(u, parts, &c, &part);
         const int j = which ? which[c] : c;
         const int4 b = boxes[j];
         const double* p = params + 6LL * j;
@@ -670,7 +679,7 @@ __global__ void __launch_bounds__(256) k_clean_stack(Image img, const int* vor, 
         const int r = render_radius(p, radius_cap);
         const double e1 = exp(p[3]), e3 = exp(p[5]);
         double* o = out + (long long)c * area;
-        for (int k = lane; k < area; k += 32) {
+        for (int k = part * 32 + lane; k < area; k += 32 * parts) {
             const int yy = k / wm, xx = k - yy * wm;
             double v = 0.0;
             if (yy < b.w && xx < b.z) {
@@ -1422,9 +1431,11 @@ int spx_clean_cells(const void* img, int dtype, double sign, int height, int wid
     if (n_out == 0 || hm == 0 || wm == 0) return SPX_OK;
     SPX_REQUIRE(img && voronoi && boxes && params && background && model && out, "null pointer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_clean_stack<<<grid_for(n_out, 8), 256, 0, s>>>(Image{img, dtype, sign, height, width}, voronoi,
-                                                       reinterpret_cast<const int4*>(boxes), params, radius_cap,
-                                                       *background, model, which, n_out, hm, wm, out);
+    // Few cells are shared out among as many warps as the chip holds, at least 32 pixels each.
+    const int parts = (int)std::max<long long>(1, std::min<long long>(((long long)hm * wm + 31) / 32, kChipWarps / n_out));
+    k_clean_stack<<<grid_for((long long)n_out * parts, 8), 256, 0, s>>>(
+        Image{img, dtype, sign, height, width}, voronoi, reinterpret_cast<const int4*>(boxes), params, radius_cap, *background,
+        model, which, n_out, parts, hm, wm, out);
     return check_launch("k_clean_stack");
 }
 
