@@ -579,22 +579,21 @@ __device__ __forceinline__ double cubic_at_inner(const double* coef, int pitch, 
     return out;
 }
 
-// The same window evaluated in FP32, the sampling precision the ray profiles use: positions, weights,
-// products and sums, from an FP32 copy of the coefficients. The weights come as six times scipy's (a third
-// fewer operations); the copy holds the coefficients over 36.
-constexpr double kQuadScale = 1.0 / 36.0;
-
-__device__ __forceinline__ void cubic_weights6_f(float t, float* w) {
-    const float s = 1.0f - t, t2 = t * t, s2 = s * s;
-    w[0] = s2 * s;
-    w[1] = fmaf(t2, fmaf(3.0f, t, -6.0f), 4.0f);
-    w[2] = fmaf(s2, fmaf(3.0f, s, -6.0f), 4.0f);
-    w[3] = t2 * t;
-}
-
+// The same window evaluated in FP32 (weights, products and sums), the sampling precision the ray
+// profiles use, from an FP32 copy of the coefficients: sample positions stay FP64 and only their
+// fractional offsets inside the window are rounded to FP32, so a sample differs from the FP64
+// evaluation by ~1e-7 relative. The caller passes the window's integer cell and the offsets.
 struct SplineWindowF {
     int fy = -1 << 30, fx = -1 << 30;
     float c[16];
+    __device__ __forceinline__ static void weights(float t, float* w) {
+        const float s = 1.0f - t;
+        const float k = 1.0f / 6.0f;
+        w[1] = (t * t * (t - 2.0f) * 3.0f + 4.0f) * k;
+        w[2] = (s * s * (s - 2.0f) * 3.0f + 4.0f) * k;
+        w[0] = s * s * s * k;
+        w[3] = 1.0f - w[0] - w[1] - w[2];
+    }
     // (iy, ix): the sample's cell in box coordinates (0 <= iy < hm, 0 <= ix < wm); the window is the
     // four float4 rows quad[(iy + a) * wm + ix], a = 0..3 (radial_quad_offset).
     __device__ __forceinline__ float at(const float4* quad, int wm, int iy, int ix, float ty, float tx) {
@@ -612,8 +611,8 @@ struct SplineWindowF {
             }
         }
         float wy[4], wx[4];
-        cubic_weights6_f(ty, wy);
-        cubic_weights6_f(tx, wx);
+        weights(ty, wy);
+        weights(tx, wx);
         float out = 0.0f;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -630,8 +629,8 @@ struct SplineWindowF {
 // SplineWindowF::at without the cached window.
 __device__ __forceinline__ float spline_sample_f(const float4* quad, int wm, int iy, int ix, float ty, float tx) {
     float wy[4], wx[4];
-    cubic_weights6_f(ty, wy);
-    cubic_weights6_f(tx, wx);
+    SplineWindowF::weights(ty, wy);
+    SplineWindowF::weights(tx, wx);
     const float4* q = quad + iy * wm + ix;
     float out = 0.0f;
 #pragma unroll
@@ -645,14 +644,6 @@ __device__ __forceinline__ float spline_sample_f(const float4* quad, int wm, int
         out = fmaf(row, wy[a], out);
     }
     return out;
-}
-
-// floor(v) for |v| < 2^22 as an int and as a float, by one addition rounded down.
-__device__ __forceinline__ int floor_f(float v, float* fl) {
-    const float magic = 12582912.0f;  // 1.5 * 2^23
-    const float t = __fadd_rd(v, magic);
-    *fl = t - magic;
-    return __float_as_int(t) - 0x4b400000;
 }
 
 // floor(y) for 0 <= y < 2^51 as an int and as a double, with FP64 additions only (no conversion
@@ -1108,13 +1099,13 @@ __device__ __forceinline__ void ray_edges64(const double* coef, int hp, int wp, 
 // FP32 sample leaves a decision elsewhere within its error bound (a sample near half height before
 // the crossing; a candidate three or more samples from the maximum level with it), ray_fp64 walks
 // the ray again with FP64 samples and that result is kept.
-// Bound: instructions (about 100,000 a cell of 24 px pitch, 128 rays of 110 samples: half of them the walk's,
-// a quarter the spline coefficients and masks, the rest the FP64 edges). With FP64 positions the walk spent 47
-// FP64 instructions a sample and 32 separate exits a warp; FP32 positions with one cheap exit test, box indices
-// without integer divisions: 29,000 such cells 4.67 -> 3.99 ms (4.17 with the position's bound taken from the longest
-// radius instead of the box's reach: more rays walked again); pitches of 14 to 60 px 12-14 % less each. Against 4.17:
-// five blocks per SM without spills measure the same (4.15), the sample taken before the validity test 4.30, the loop
-// unrolled by two 4.60.
+// Bound: instructions (half of a cell's are the walk's at 24 px pitch, 128 rays of 110 samples; a quarter the
+// spline coefficients and masks, the rest the FP64 edges). One cheap exit test instead of the mask's weights wherever
+// a pixel square is not whole (the lanes end in 32 different places) and box indices without integer divisions:
+// 29,000 such cells 4.67 -> 4.06 ms, 5-20 % less from 14 to 130 px pitch, 1-4 % at 200 to 500 px. Positions stay FP64:
+// with FP32 ones the walk takes 3.99 ms there, but their error bound sends more rays to the FP64 re-walk the larger
+// and smoother a cell is (noise-free cells of 40 and 60 px 1.0 and 1.9 ms against 3.9 and 7.5, 500 px 11.2
+// against 18).
 template <bool kSmooth, int kRays>
 __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
     const double* cleaned, const int* vor, const int4* boxes, const int* which, int n, int hm, int wm, int W,
@@ -1226,7 +1217,7 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
         }
         for (int k = tid; k < area_px; k += kRadialThreads) {
             int yy, xx;
-                by_wm(k, &yy, &xx);
+            by_wm(k, &yy, &xx);
             emask[k] = mask[k] && yy > 0 && xx > 0 && yy < hm - 1 && xx < wm - 1 && mask[k - wm] && mask[k + wm] &&
                        mask[k - 1] && mask[k + 1];
         }
@@ -1247,33 +1238,18 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
             int yy, xx;
             by_wm(k, &yy, &xx);
             const double* q = coef + (yy + kPad - 1) * dp + (xx + kPad - 1);
-            const float4 f = make_float4((float)(q[0] * kQuadScale), (float)(q[1] * kQuadScale),
-                                         (float)(q[2] * kQuadScale), (float)(q[3] * kQuadScale));
+            const float4 f = make_float4((float)q[0], (float)q[1], (float)q[2], (float)q[3]);
             quad[k] = f;
             cmax = fmaxf(cmax, fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
         }
-        // A sample's FP32 position is within perr = (4 X + 2) 2^-24 pixels of the FP64 one in each axis (X: the box's
-        // farthest side from the centre, plus one; the roundings of step, radius, direction, sum and centre). The
-        // window weights are non-negative and sum to one per axis, their derivatives' magnitudes to at most 1.5, so a
-        // sample is within about 45 ulps of cmax (coefficient and weight roundings, 20 FMAs) + 3 perr cmax of the FP64
-        // one; tol keeps a margin (2^-17 cmax + 4 perr cmax). Also orders the quad writes before the rays read them.
+        // The window weights are non-negative and sum to one per axis, so an FP32 sample is within about
+        // 45 ulps of cmax of the FP64 one (coefficient, offset and weight roundings, 20 FMAs); tol keeps
+        // a margin of nearly 3 (2^-17 cmax). Also orders the quad writes before the rays read them.
         if (tid == 0) s_nq = 0;  // before the barrier in cta_max; read after the barrier that follows the rays
-        const double reach = fmax(fmax(cx, (double)(wm - 1) - cx), fmax(cy, (double)(hm - 1) - cy)) + 1.0;
-        const float perr = (4.0f * (float)reach + 2.0f) * 5.9604644775390625e-08f;
-        const float tol = (float)cta_max((double)cmax, red + 28) * 36.0f * (7.62939453125e-06f + 4.0f * perr);
-        const float inner = 0.5f - 2.0f * perr;
-        const float stepf = (float)radial_step;
-        const int icy = (int)floor(cy), icx = (int)floor(cx);
-        const float fcy = (float)(cy - icy), fcx = (float)(cx - icx);
+        const float tol = (float)cta_max((double)cmax, red + 28) * 7.62939453125e-06f;
         const double half = peak / 2.0;
         int j_min = 2;  // first gradient candidate: j >= 2 and j * step >= thr
         while ((double)j_min * radial_step < thr) ++j_min;
-        // Whether the square [iy, iy + 1] x [ix, ix + 1] lies inside the eroded cell.
-        auto square = [&](int iy, int ix) -> bool {
-            if constexpr (kRays != 0) return full[iy * wm + ix];
-            const uint8_t* q = emask + iy * wm + ix;
-            return iy + 1 < hm && ix + 1 < wm && q[0] && q[1] && q[wm] && q[wm + 1];
-        };
         int found_h = 0, found_g = 0;
         for (int ray = tid; ray < n_angles; ray += kRadialThreads) {
             double edge_h = dnan(), edge_g = dnan();
@@ -1281,8 +1257,8 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
             if (peak > 0.0) {
                 const double ang = (double)ray * (2.0 * kPi / n_angles);
                 const double ux = trig ? trig[2 * ray] : cos(ang), uy = trig ? trig[2 * ray + 1] : sin(ang);
-                // Positions and samples are FP32 and so are the walk's decisions on them; where a ray ends is
-                // decided as in FP64, and the edges are computed from FP64 samples at the decisive positions.
+                // Samples are FP32 (SplineWindowF) and the walk's decisions are FP32; the edges are then
+                // computed from FP64 samples at the decisive positions.
                 float h1 = 0, h2 = 0, h3 = 0;  // p[k-1] .. p[k-3]
                 int kc = -1;                   // first FP32 crossing: p[kc-1] >= half > p[kc]
                 bool amb_h = false;            // a sample up to kc within tol of half height
@@ -1293,42 +1269,35 @@ __global__ void __launch_bounds__(kRadialThreads, 6) k_radial_cd(
                 int best_j = -1, first_invalid = n_radii;
                 const float halff = (float)half;
                 SplineWindowF win;
-                const float uyf = (float)uy, uxf = (float)ux;
-                float kf = 0.0f;  // k as a float (exact), so r = k * step needs no conversion
+                int mfy = -1 << 30, mfx = -1 << 30;  // mask cell of the last sample and whether all
+                bool mfull = false;                   // four of its corners are in the eroded cell
+                const double ymax = (double)(hm - 1), xmax = (double)(wm - 1);
                 const int j_first = j_min + 2;
-                for (int k = 0; k < n_radii; ++k, kf += 1.0f) {
-                    const float rf = kf * stepf;
-                    const float yo = fmaf(uyf, rf, fcy), xo = fmaf(uxf, rf, fcx);
-                    float fly, flx;
-                    int iy = icy + floor_f(yo, &fly), ix = icx + floor_f(xo, &flx);
-                    float ty = yo - fly, tx = xo - flx;
-                    // Valid without doubt: all four corners of the pixel square in the eroded cell, and the
-                    // position farther from the square's edges than it can be wrong.
-                    const bool in = (unsigned)iy < (unsigned)hm && (unsigned)ix < (unsigned)wm;
-                    const bool whole = in && square(iy, ix);
-                    const float off = fmaxf(fabsf(ty - 0.5f), fabsf(tx - 0.5f));
-                    if (!(whole && off <= inner)) {
-                        // Outside without doubt: a missing corner's weight is at least (0.01 - perr)^2.
-                        if (in && !whole && off <= 0.49f && inner >= 0.49f) {
-                            first_invalid = k;
-                            break;
+                double kd = 0.0;  // k as a double (exact), so r = k * step needs no conversion
+                for (int k = 0; k < n_radii; ++k, kd += 1.0) {
+                    const double r = kd * radial_step;
+                    const double x = __dadd_rn(cx, __dmul_rn(ux, r)), y = __dadd_rn(cy, __dmul_rn(uy, r));
+                    if (!(y >= 0.0 && y <= ymax && x >= 0.0 && x <= xmax)) { first_invalid = k; break; }
+                    double fyd, fxd;
+                    const int iy = floor_nonneg(y, &fyd), ix = floor_nonneg(x, &fxd);
+                    const float ty = (float)(y - fyd), tx = (float)(x - fxd);
+                    bool whole;  // all four corners of the pixel square are in the eroded cell
+                    if constexpr (kRays == 2) {
+                        whole = full[iy * wm + ix];
+                    } else {
+                        if (iy != mfy || ix != mfx) {
+                            mfy = iy;
+                            mfx = ix;
+                            const uint8_t* q = emask + iy * wm + ix;
+                            mfull = iy + 1 < hm && ix + 1 < wm && q[0] && q[1] && q[wm] && q[wm + 1];
                         }
-                        // The FP64 position decides.
-                        const double r = (double)k * radial_step;
-                        const double x = __dadd_rn(cx, __dmul_rn(ux, r)), y = __dadd_rn(cy, __dmul_rn(uy, r));
-                        if (!(y >= 0.0 && y <= (double)(hm - 1) && x >= 0.0 && x <= (double)(wm - 1))) {
-                            first_invalid = k;
-                            break;
-                        }
-                        double fyd, fxd;
-                        iy = floor_nonneg(y, &fyd);
-                        ix = floor_nonneg(x, &fxd);
-                        if (!(square(iy, ix) || inside_bytes(emask, hm, wm, y, x))) {
-                            first_invalid = k;
-                            break;
-                        }
-                        ty = (float)(y - fyd);
-                        tx = (float)(x - fxd);
+                        whole = mfull;
+                    }
+                    // A missing corner ends the ray where it weighs 1e-4 or more (the mask's spline has to reach
+                    // 1 - 1e-8); nearer to the square's edges the weights decide.
+                    if (!whole && (fmaxf(fabsf(ty - 0.5f), fabsf(tx - 0.5f)) <= 0.49f || !inside_bytes(emask, hm, wm, y, x))) {
+                        first_invalid = k;
+                        break;
                     }
                     float p;
                     if constexpr (kRays == 2) p = spline_sample_f(quad, wm, iy, ix, ty, tx);

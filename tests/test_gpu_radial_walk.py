@@ -65,3 +65,10 @@ def test_edges_match_oracle(h, w, step, form):
         got, want = b["edge_px"].cpu().numpy(), ref[name]["edge_px"]
         np.testing.assert_array_equal(np.isnan(got), np.isnan(want), err_msg=name)
         np.testing.assert_allclose(got, want, rtol=0, atol=1e-7, err_msg=name)
+
+
+@pytest.mark.parametrize("h,w,step", [(40, 40, 0.1), (131, 140, 0.37), (200, 211, 0.1)])
+def test_edges_of_large_cells_match_oracle(h, w, step):
+    """Boxes in the global scratch and noise-free cells, where most gradient maxima are walked again in FP64. A 200 px cell's
+    decreases differ by 1e-6 of the signal a step around their maximum, so the bound above holds here too."""
+    test_edges_match_oracle(h, w, step, 2)
