@@ -2725,9 +2725,8 @@ static int launch_radial(const double* cleaned, const int* voronoi, const int* b
     double* scratch = nullptr;
     int blocks;
     if (smem) {
-        if (smem + 2 * kTrigMax * sizeof(double) > 48 * 1024)  // with the static cos / sin table
-            SPX_CUDA(cudaFuncSetAttribute(k_radial_cd<kSmooth, kRays>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+        // (Always: the kernel's static arrays count towards the 48 KB that need no attribute.)
+        SPX_CUDA(cudaFuncSetAttribute(k_radial_cd<kSmooth, kRays>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_radial_cd<kSmooth, kRays>, kRadialThreads,
                                                                smem));
