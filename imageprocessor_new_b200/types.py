@@ -76,12 +76,14 @@ class CDResult:
 
     def __post_init__(self):
         """Mean original intensity over each full Voronoi cell, without fill."""
-        # Bin 0 takes the pixels of no cell (label -1): the sums of the others run over the same pixels in the
+        # Bin 0 takes the pixels of no cell (negative labels): the sums of the others run over the same pixels in the
         # same order as over the assigned ones alone, without gathering them.
-        labels = np.asarray(self.cell_labels)
-        totals = np.bincount(
-            (labels + 1).ravel(), weights=np.asarray(self.image, dtype=np.float64).ravel(), minlength=len(self.seeds_xy) + 1,
-        )[1:]
+        image = np.asarray(self.image, dtype=np.float64)
+        bins = np.maximum(self.cell_labels, np.int64(-1))
+        if image.shape != bins.shape:
+            raise IndexError(f"image of shape {image.shape} does not match cell_labels of shape {bins.shape}")
+        bins += 1
+        totals = np.bincount(bins.ravel(), weights=image.ravel(), minlength=len(self.seeds_xy) + 1)[1:]
         self.mean_intensity = np.divide(
             totals, self.cell_areas_px2,
             out=np.full(len(self.seeds_xy), np.nan), where=self.cell_areas_px2 > 0,
