@@ -20,6 +20,7 @@ plain initial fit as production; each "ok" cell gives one (patch, fit) example.
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass
 from pathlib import Path
 
@@ -323,8 +324,16 @@ def pages_cells(pages, *, area_min: int = 10, area_max: int = 2000, pad: int = 3
         while end < len(pages) and (end == at or px + pages[end].numel() <= _TOGETHER_PIXELS):
             px += pages[end].numel()
             end += 1
-        yield from _cells_together(pages[at:end], int(area_min), int(area_max), pad)
+        yield from _cells_together(pages[at:end], *_area_limits(area_min, area_max), pad)
         at = end
+
+
+def _area_limits(area_min, area_max) -> tuple[int, int]:
+    """The 32-bit limits that keep the areas a with area_min <= a <= area_max, for any real limits."""
+    most = 2**31 - 1
+    if not (area_min <= most and area_max >= 0 and area_min <= area_max):  # (NaN keeps nothing)
+        return 1, 0
+    return math.ceil(max(area_min, 0)), math.floor(min(area_max, most))
 
 
 def _cells_together(pages, area_min: int, area_max: int, pad: int):

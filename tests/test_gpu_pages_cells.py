@@ -35,3 +35,19 @@ def test_pages_cells(monkeypatch):
                          (c.seeds_d, one.seeds_d)):
                 assert torch.equal(x, y)
     assert alone[2].n == 0
+
+
+@pytest.mark.parametrize("limits", [(20.5, 30.5), (20, float("inf")), (float("-inf"), 300), (0, 2**40), (-3, 25.0),
+                                    (2**33, 2**34), (40.2, 40.8), (300, 20), (float("nan"), 300), (20, float("nan")),
+                                    (np.float32(20.5), np.int64(300))])
+def test_area_limits_are_compared_as_given(limits):
+    from imageprocessor_new_b200 import _device as dev, synthetic, warmstart as ws
+    from imageprocessor_new_b200.cd import _segment
+
+    page = dev.upload(synthetic.page_square(1, shape=(160, 200)).image)
+    comp, _ = _segment(page, "otsu", False)
+    area = comp.stats.cpu().numpy()[1:, 4]
+    assert len(np.unique(area)) > 3
+    got = ws.page_cells(page, area_min=limits[0], area_max=limits[1])
+    keep = (area >= limits[0]) & (area <= limits[1])
+    np.testing.assert_array_equal(got.rows[:, 4:6], comp.centroids.cpu().numpy()[1:][keep])
