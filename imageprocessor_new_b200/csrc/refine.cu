@@ -286,28 +286,56 @@ __device__ __forceinline__ bool in_mask(const int* labels, int W, const Roi& r, 
     return labels[(long long)(r.y0 + yy) * W + (r.x0 + xx)] == r.label;
 }
 
+// fn(y, x) for every mask pixel of a ROI in global memory, pixel k on lane k mod 32, kAhead labels in flight (1: the
+// plain loop, unrolled as the compiler will). Bound: latency of one warp per ROI. Where the loop stands beside the
+// staged path the compiler no longer unrolls it: NONE on a 200 px ROI of an integer image 154 us in a kernel of its
+// own, 219 us beside the staged path, 100 us with eight in flight; log-quadratic (with two in its own loop, as its
+// registers allow) 934, 1032 and 908 us, 1,000 ROIs of 66 px 143, 153 and 143 us. The weighted and edge refiners keep the
+// plain loop: there more in flight costs the staged path registers (40,000 ROIs of 20 px 98 -> 104 us).
+template <int kAhead, class F>
+__device__ __forceinline__ void each_mask_pixel(const int* labels, int W, const Roi& r, int lane, F&& fn) {
+    const int P = r.w * r.h;
+    if constexpr (kAhead == 1) {
+        for (int k = lane; k < P; k += 32) {
+            const int yy = k / r.w, xx = k % r.w;
+            if (in_mask(labels, W, r, yy, xx)) fn(yy, xx);
+        }
+    } else {
+        for (int k0 = lane; k0 < P; k0 += 32 * kAhead) {
+            int yy[kAhead], xx[kAhead], lab[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int k = min(k0 + 32 * u, P - 1);
+                yy[u] = k / r.w;
+                xx[u] = k - yy[u] * r.w;
+                lab[u] = labels[(long long)(r.y0 + yy[u]) * W + (r.x0 + xx[u])];
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (lab[u] == r.label && k0 + 32 * u < P) fn(yy[u], xx[u]);
+        }
+    }
+}
+
 // Mask pixel count and exact integer coordinate sums (ROI-local), plus the mask bbox.
 struct MaskSums {
     long long n, sx, sy;
     int xmin, xmax, ymin, ymax;
 };
 
+template <int kAhead>
 __device__ MaskSums mask_sums(const int* labels, int W, const Roi& r, int lane) {
     long long n = 0, sx = 0, sy = 0;
     int xmin = 0x7fffffff, xmax = -1, ymin = 0x7fffffff, ymax = -1;
-    const int P = r.w * r.h;
-    for (int k = lane; k < P; k += 32) {
-        const int yy = k / r.w, xx = k % r.w;
-        if (in_mask(labels, W, r, yy, xx)) {
-            ++n;
-            sx += xx;
-            sy += yy;
-            xmin = min(xmin, xx);
-            xmax = max(xmax, xx);
-            ymin = min(ymin, yy);
-            ymax = max(ymax, yy);
-        }
-    }
+    each_mask_pixel<kAhead>(labels, W, r, lane, [&](int yy, int xx) {
+        ++n;
+        sx += xx;
+        sy += yy;
+        xmin = min(xmin, xx);
+        xmax = max(xmax, xx);
+        ymin = min(ymin, yy);
+        ymax = max(ymax, yy);
+    });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         n += __shfl_xor_sync(0xffffffffu, n, o);
@@ -480,6 +508,8 @@ struct StagedPixels {
     __device__ __forceinline__ double value(int yy, int xx) const { return (double)s.px[yy * s.w + xx]; }
 };
 
+// (kSums, kAhead: labels in flight in the mask's sums and in each.)
+template <int kSums, int kAhead>
 struct GlobalPixels {
     const void* img;
     int dtype;
@@ -487,16 +517,13 @@ struct GlobalPixels {
     int W;
     Roi r;
     double* keys;
-    __device__ __forceinline__ MaskSums sums(int lane) const { return mask_sums(labels, W, r, lane); }
+    __device__ __forceinline__ MaskSums sums(int lane) const { return mask_sums<kSums>(labels, W, r, lane); }
     __device__ __forceinline__ double background(int lane) const {
         return border_median(img, dtype, W, r, keys, lane);
     }
     template <class F>
     __device__ __forceinline__ void each(int lane, F&& fn) const {
-        for (int k = lane; k < r.w * r.h; k += 32) {
-            const int yy = k / r.w, xx = k % r.w;
-            if (in_mask(labels, W, r, yy, xx)) fn(yy, xx, value(yy, xx));
-        }
+        each_mask_pixel<kAhead>(labels, W, r, lane, [&](int yy, int xx) { fn(yy, xx, value(yy, xx)); });
     }
     __device__ __forceinline__ double value(int yy, int xx) const {
         return load_px(img, dtype, (long long)(r.y0 + yy) * W + (r.x0 + xx));
@@ -897,6 +924,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 k_refine(const void* img, int dtype, int H, int W, const int* labels, const int* rows,
          const uint8_t* methods, int n, const int* n_dev, int fill, int pad, double* centers) {
     constexpr bool kInteger = !std::is_void<Px>::value;
+    constexpr int kSums = kInteger && M == SPX_REFINE_NONE ? 8 : 1;
     // Integer images: the staged ROI, or the general path's 256-bin histogram; the edge refiner's profiles.
     // Others: the general path's sort keys.
     __shared__ double keys[kWarpsPerBlock][kInteger ? kRoiSide * kRoiSide / 4 : kSortCap];
@@ -926,9 +954,9 @@ k_refine(const void* img, int dtype, int H, int W, const int* labels, const int*
                                                list[warp]},
                                   r, prof[warp], lane, &cx, &cy);
                 else
-                    refine_roi<M>(GlobalPixels{img, dtype, labels, W, r, keys[warp]}, r, prof[warp], lane, &cx, &cy);
+                    refine_roi<M>(GlobalPixels<kSums, 1>{img, dtype, labels, W, r, keys[warp]}, r, prof[warp], lane, &cx, &cy);
             } else {
-                refine_roi<M>(GlobalPixels{img, dtype, labels, W, r, keys[warp]}, r, prof[warp], lane, &cx, &cy);
+                refine_roi<M>(GlobalPixels<kSums, 1>{img, dtype, labels, W, r, keys[warp]}, r, prof[warp], lane, &cx, &cy);
             }
         }
         if (lane == 0) {
@@ -942,10 +970,12 @@ k_refine(const void* img, int dtype, int H, int W, const int* labels, const int*
 // The log-quadratic refiner. A warp takes its blobs one after another as far as their sums, and solves up
 // to kLogquadBatch of them together, one per lane: the 6 x 6 elimination with its divisions is a serial chain
 // that all lanes of a warp would otherwise repeat for every single blob (more than half of the kernel).
+// Registers for six blocks an SM with integer images; the sort keys of the others leave room for four (with six the
+// 27 sums spill: 20,000 ROIs of 42 px of a float image 1158 us one blob after another, 1213 spilt, now 1048).
 constexpr int kLogquadBatch = 16;
 
 template <typename Px>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, std::is_void<Px>::value ? 4 : 6)
 k_refine_logquad(const void* img, int dtype, int H, int W, const int* labels, const int* rows, const uint8_t* methods,
                  int n, const int* n_dev, int fill, int pad, double* centers) {
     constexpr bool kInteger = !std::is_void<Px>::value;
@@ -992,7 +1022,7 @@ k_refine_logquad(const void* img, int dtype, int H, int W, const int* labels, co
                                        r, lane, out, &degenerate);
                 }
             }
-            if (!staged) fit = logquad_sums(GlobalPixels{img, dtype, labels, W, r, keys[warp]}, r, lane, out, &degenerate);
+            if (!staged) fit = logquad_sums(GlobalPixels<8, 2>{img, dtype, labels, W, r, keys[warp]}, r, lane, out, &degenerate);
         }
         if (lane == 0) {
             if (fit) held[warp][waiting] = LogquadBlob{blob, r.x0, r.y0, r.w, r.h, degenerate};

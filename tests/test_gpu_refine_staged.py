@@ -85,3 +85,38 @@ def test_rows_past_a_device_count_are_nan():
         c = out.cpu().numpy()
         assert np.isnan(c[n // 2:]).all()
         assert np.isfinite(c[: n // 2]).any() and not (c == -7.0).any()
+
+
+@pytest.mark.parametrize("w,h", [(33, 1), (7, 41), (31, 33), (64, 64), (65, 63), (190, 77)])
+@pytest.mark.parametrize("refine", ["none", "weighted", "logquad", "edge_gradmoment"])
+def test_large_rois_take_the_same_pixels_in_the_same_order(refine, w, h):
+    """ROIs that are not staged, of integer images against the same image as float64 (the same bits) and, for the mean of
+    the mask, against NumPy's exact one: pixel counts on either side of a round of 32 lanes with several labels in
+    flight, masks with holes, ROIs clipped by the image."""
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    rng = np.random.default_rng(w * h)
+    H, W = h + 4, w + 5
+    yy, xx = np.mgrid[:H, :W]
+    r2 = ((yy - 0.48 * H) / (0.45 * H)) ** 2 + ((xx - 0.53 * W) / (0.45 * W)) ** 2
+    m = (r2 <= 1.2) & (rng.random((H, W)) < 0.9)
+    m[:2], m[-2:], m[:, :2], m[:, -3:] = False, False, False, False
+    m[2, 2] = m[h + 1, w + 1] = True
+    img = np.clip(np.rint(100 + 120 * np.exp(-r2) + rng.normal(0, 2, (H, W))), 0, 255)
+    lab_d, rows_d = dev.upload(np.where(m, 7, 3).astype(np.int32)), dev.upload(np.array([[2, 2, w, h, 7]], np.int32))
+    code = _lib.REFINE_CODES[refine]
+    meth_d = dev.upload(np.full(1, code, np.uint8))
+    for pad in (0, 9):
+        got = []
+        for dtype in ("uint8", "uint16", "float32", "float64"):
+            img_d, out = dev.upload(img.astype(dtype)), dev.upload(np.zeros((1, 2)))
+            _lib.call("spx_refine_selected", img_d.data_ptr(), dev.dtype_code(img_d), H, W, lab_d.data_ptr(),
+                      rows_d.data_ptr(), meth_d.data_ptr(), 1, None, pad, code, out.data_ptr(), dev.stream_ptr())
+            got.append(out.cpu().numpy())
+        for g in got[:-1]:
+            np.testing.assert_array_equal(g, got[-1])
+        if refine == "none":
+            y0, x0 = max(0, 2 - pad), max(0, 2 - pad)
+            ys, xs = np.nonzero(m[y0:, x0:])
+            np.testing.assert_array_equal(got[-1], [[x0 + xs.sum() / len(xs), y0 + ys.sum() / len(ys)]])
