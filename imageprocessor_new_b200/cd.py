@@ -769,14 +769,15 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
         seconds["result"] = time.perf_counter() - start
         seconds["total"] = time.perf_counter() - started
         return result
-    # The reported cells' labels and areas on the device, from the Voronoi labels of all cells.
-    remap = np.full(max(len(rows), 1), -1, dtype=np.int32)
-    remap[report] = np.arange(nr, dtype=np.int32)
-    remap_d = dev.upload(remap)
-    flat = c.voronoi.view(-1)
-    labels_out = remap_d.index_select(0, flat) if len(rows) else torch.full_like(flat, -1)
-    areas = torch.bincount(labels_out.add(1), minlength=nr + 1)[1:].cpu().numpy()
-    cell_labels = dev.download(labels_out.view(shape))
+    if nr:
+        # The reported cells' labels and areas on the device, from the Voronoi labels of all cells.
+        remap = np.full(len(rows), -1, dtype=np.int32)
+        remap[report] = np.arange(nr, dtype=np.int32)
+        labels_out = dev.upload(remap).index_select(0, c.voronoi.view(-1))
+        areas = torch.bincount(labels_out.add(1), minlength=nr + 1)[1:].cpu().numpy()
+        cell_labels = dev.download(labels_out.view(shape))
+    else:  # (the passes above cost such a page 0.15 to 0.6 ms: 403 x 1352 px 3.8 -> 4.6 ms as a whole)
+        areas, cell_labels = np.zeros(0, np.int64), np.full(shape, -1, dtype=np.int32)
     params_global = state.params.copy()
     params_global[:, 1:3] += c.origins
     deblend_model = {"params": params_global, "report": report.astype(np.int64), "tile_px": int(state.tile_px)}
@@ -786,7 +787,7 @@ def _measure_cds(img, *, methods, threshold, invert, area_min, area_max, pad, n_
         rois, masks = np.empty((nr, 0, 0)), np.empty((nr, 0, 0), bool)
     else:
         rois = dev.download(cleaned)
-        masks = _mask_stack(c, report)
+        masks = _mask_stack(c, report) if nr else np.zeros(rois.shape, bool)
     result = CDResult(
         image=dev.download(img_d) if isinstance(img, torch.Tensor) else img.copy(),
         binary=np.zeros(shape, bool) if comp is None else dev.download(comp.labels > 0),

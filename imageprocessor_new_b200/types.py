@@ -78,12 +78,16 @@ class CDResult:
         """Mean original intensity over each full Voronoi cell, without fill."""
         # Bin 0 takes the pixels of no cell (negative labels): the sums of the others run over the same pixels in the
         # same order as over the assigned ones alone, without gathering them.
-        image = np.asarray(self.image, dtype=np.float64)
-        bins = np.maximum(self.cell_labels, np.int64(-1))
-        if image.shape != bins.shape:
-            raise IndexError(f"image of shape {image.shape} does not match cell_labels of shape {bins.shape}")
+        image, labels = np.asarray(self.image), np.asarray(self.cell_labels)
+        if image.shape != labels.shape:
+            raise IndexError(f"image of shape {image.shape} does not match cell_labels of shape {labels.shape}")
+        if not len(self.seeds_xy) and not (labels >= 0).any():
+            self.mean_intensity = np.zeros(0)
+            return
+        bins = np.maximum(labels, np.int64(-1))
         bins += 1
-        totals = np.bincount(bins.ravel(), weights=image.ravel(), minlength=len(self.seeds_xy) + 1)[1:]
+        totals = np.bincount(bins.ravel(), weights=np.asarray(image, dtype=np.float64).ravel(),
+                             minlength=len(self.seeds_xy) + 1)[1:]
         self.mean_intensity = np.divide(
             totals, self.cell_areas_px2,
             out=np.full(len(self.seeds_xy), np.nan), where=self.cell_areas_px2 > 0,
