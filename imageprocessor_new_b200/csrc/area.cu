@@ -19,8 +19,8 @@
 // values, so each later step evaluates only the units that can hold what it looks for.
 //
 // Measured on one B200 against the dense kernels: the five tail methods of 4,032 windows of 59 px (both
-// passes) 80.3 -> 6.7 ms; half_area and half_area_min + _min_avg of the 7,225 cells of a 2047 x 2050 page
-// (24 px) 5.47 -> 1.37 ms.
+// passes) 80.3 -> 6.9 ms; half_area and half_area_min + _min_avg of the 7,225 cells of a 2047 x 2050 page
+// (24 px) 5.47 -> 1.42 ms.
 
 #include <algorithm>
 
@@ -209,10 +209,13 @@ __device__ __forceinline__ float key_float(unsigned k) {
     return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k);
 }
 
-// The highest masked sub-pixel (first in row-major order on ties; -inf and 0 when the mask is empty) on
-// every thread, and the units' upper bounds.
+// The highest masked sub-pixel's value and, in top->y, its place (-inf and 0 when the mask is empty), on every
+// thread, and the units' upper bounds. top->x: the first sub-pixel in row-major order that reaches it to rounding (a
+// margin of 2^-48, twice the sums' error): equal peaks of a cell (isolated pixels of one value, mirrored holes) differ
+// in the last bits of the recursion's sums, and the reference takes the first of equal ones. It is looked up over the
+// few units that reach the peak (2-3 % of the kernels).
 template <int NT>
-__device__ void area_peak(const AreaCta<NT>& h, double* s_red, int* s_ired, double* top_v, int* top) {
+__device__ void area_peak(const AreaCta<NT>& h, double* s_red, int* s_ired, double* top_v, int2* top) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = h.g.RW;
     double best = -INFINITY;
     int best_i = 0x7fffffff;
@@ -256,8 +259,27 @@ __device__ void area_peak(const AreaCta<NT>& h, double* s_red, int* s_ired, doub
             best = s_red[q];
             best_i = s_ired[q];
         }
+    __syncthreads();
+    const double reach = best - 0x1p-48 * best;
+    int first = best_i;
+    if (best > 0.0 && isfinite(best))
+        for (int ky = warp; ky < h.g.hm; ky += NT / 32)
+            for (int w = 0; w < RW; ++w) {
+                if ((double)h.unit[ky * RW + w] < reach) continue;
+                const int X = min(w * 32 + lane, h.g.Wb - 1);
+                double v[4];
+                unit_values(h.coef, h.g.cp, ky, X, v);
+                if (!((h.pmask[ky * RW + w] >> lane) & 1u)) continue;
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (v[p] >= reach) first = min(first, (kF * ky + p) * h.g.Wb + X);
+            }
+    first = __reduce_min_sync(0xffffffffu, first);
+    if (lane == 0) s_ired[warp] = first;
+    __syncthreads();
+    for (int q = 0; q < NT / 32; ++q) first = min(first, s_ired[q]);
     *top_v = best;
-    *top = best_i == 0x7fffffff ? 0 : best_i;
+    *top = best_i == 0x7fffffff ? make_int2(0, 0) : make_int2(first, best_i);
     __syncthreads();
 }
 
@@ -385,7 +407,7 @@ struct AreaOptions {
 // whatever the order: centroid SX / n, spreads (n SXX - SX^2) / n^2.
 template <int NT>
 __device__ void area_output(const AreaCta<NT>& h, const AreaOptions& o, const MethodOut& out, int i, double b,
-                            double peak, double cut, double steepest, int top, const AreaPlace& at,
+                            double peak, double cut, double steepest, int2 top, const AreaPlace& at,
                             unsigned long long* s_mom, double* s_red) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hm = h.g.hm, Hb = h.g.Hb, Wb = h.g.Wb, RW = h.g.RW;
@@ -414,12 +436,10 @@ __device__ void area_output(const AreaCta<NT>& h, const AreaOptions& o, const Me
             }
         }
     __syncthreads();
-    const int top_row = top / Wb;
-    if (tid == 0) {
-        const int X = top % Wb;
-        const uint32_t bitv = 1u << (X % 32);
-        if (h.above[top_row * RW + X / 32] & bitv) h.reg[top_row * RW + X / 32] = bitv;
-    }
+    // (A threshold within the margin of the peak can leave the first place below it.)
+    auto is_above = [&](int t) { return (h.above[t / Wb * RW + t % Wb / 32] >> (t % Wb % 32)) & 1u; };
+    const int start = is_above(top.x) ? top.x : top.y, top_row = start / Wb;
+    if (tid == 0 && is_above(start)) h.reg[top_row * RW + start % Wb / 32] = 1u << (start % Wb % 32);
     __syncthreads();
     // Grown from the highest sub-pixel one 8-neighbour ring per step until it stops changing; step s + 1
     // only computes the rows within s + 1 of the start.
@@ -608,7 +628,7 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_half_area_spline(const __grid_
         }
         spline_coefs(h);
         double top_v;
-        int top;
+        int2 top;
         area_peak(h, s_red, s_ired, &top_v, &top);
         const AreaPlace at{(double)c.box.x, (double)c.box.y, dnan(), dnan()};
         // The averaged peak reads the list that the bit planes of an output replace.
@@ -727,7 +747,7 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_tail_area_spline(const __grid_
             }
             spline_coefs(h);
             double top_v;
-            int top;
+            int2 top;
             area_peak(h, s_red, s_ired, &top_v, &top);
             double peak = -1.0;
             if (t.o.n_top <= h.g.Hb * h.g.Wb)

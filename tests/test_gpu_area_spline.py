@@ -142,3 +142,39 @@ def test_tail_area_spline_matches_the_dense_operators(side, n_top, outlines):
         torch.cuda.synchronize()
     for a, b in zip(got, want):
         _same(a, b)
+
+
+@pytest.mark.parametrize("size", [11, 24, 31, 33, 36])
+def test_the_first_of_equal_peaks_is_taken(size):
+    """Two equal isolated pixels, mirrored in the cell: equal peaks in exact arithmetic, whatever the last bits of either
+    side's sums. The region is the first one's in row-major order, in cells and in windows."""
+    import torch
+
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    lo, hi = 2, size - 3
+    pairs = [((y, lo), (y, hi)) for y in range(2, size - 2)] + [((lo, x), (hi, x)) for x in range(2, size - 2)]
+    pairs += [((lo, lo), (hi, hi)), ((lo, hi), (hi, lo))]
+    n = len(pairs)
+    cells = np.zeros((n, size, size))
+    for i, (a, b) in enumerate(pairs):
+        cells[i][a] = cells[i][b] = 37.0 + 3.3 * i
+    vor = np.repeat(np.arange(n, dtype=np.int32), size)[:, None] * np.ones((1, size), np.int32)
+    boxes = np.column_stack((np.zeros(n), np.arange(n) * size, np.full(n, size), np.full(n, size))).astype(np.int32)
+    roi, vor_d, boxes_d = dev.upload(cells), dev.upload(np.ascontiguousarray(vor)), dev.upload(boxes)
+    (single, ss), (avg, sa) = _outputs(n, 13), _outputs(n, 13)
+    _lib.call("spx_half_area_spline_cd", roi.data_ptr(), vor_d.data_ptr(), boxes_d.data_ptr(), None, n, size, size, size,
+              ANGLES, 0.5, 0, 16, 1, ss, sa, dev.stream_ptr())
+    win = dev.upload(cells.astype(np.float32))
+    ones = dev.upload(np.ones((n, size, size), np.uint8))
+    org = dev.upload(np.zeros((n, 2), np.int32))
+    norm, sn = _outputs(n, 13)
+    _lib.call("spx_tail_area_spline_cd", win.data_ptr(), ones.data_ptr(), ones.data_ptr(), ones.data_ptr(),
+              org.data_ptr(), org.data_ptr(), n, size, ANGLES, 0.5, 16, 1, None, None, sn, None, None, None,
+              dev.stream_ptr())
+    torch.cuda.synchronize()
+    want = np.array([(x, y) for (y, x), _ in pairs], float)
+    for out in (single, avg):
+        np.testing.assert_allclose(out["center_local"].cpu().numpy(), want, atol=0.3)
+    np.testing.assert_allclose(norm["centers"].cpu().numpy(), want, atol=0.3)
