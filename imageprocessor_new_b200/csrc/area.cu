@@ -543,7 +543,7 @@ __device__ void area_output(const AreaCta<NT>& h, const AreaOptions& o, const Me
                     cur, RW, h.tmp, s_red, at);
 }
 
-// Rank of the middle values of n values v (ties by position); *m = their mean, on every thread.
+// Mean of the middle value(s) by rank (ties by position) of n values, none of them NaN; NaN if there are none.
 template <int NT>
 __device__ double cta_median(const double* v, int n, double* s_mid) {
     const int k1 = (n - 1) / 2, k2 = n / 2;
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_half_area_spline(const __grid_
                                h.pixel(y, x - 1) && h.pixel(y, x + 1);
             if (!inner) {
                 const double v = c.roi[k];
-                if (a.median) ring[atomicAdd(&s_n[0], 1)] = v;
+                if (a.median && !isnan(v)) ring[atomicAdd(&s_n[0], 1)] = v;
                 lmin = fmin(lmin, v);
             }
         }
@@ -737,7 +737,8 @@ __global__ void __launch_bounds__(NT, 640 / NT) k_tail_area_spline(const __grid_
                 // nanmedian of the level pixels inside the window (NaN if none).
                 double* lv = h.coef;
                 for (int k = tid; k < area; k += NT)
-                    if (t.inside[base + k] && t.levelm[base + k]) lv[atomicAdd(&s_n[0], 1)] = (double)t.cells[base + k];
+                    if (t.inside[base + k] && t.levelm[base + k] && !isnan(t.cells[base + k]))
+                        lv[atomicAdd(&s_n[0], 1)] = (double)t.cells[base + k];
                 __syncthreads();
                 b = cta_median<NT>(lv, s_n[0], s_mid);
             }

@@ -1947,7 +1947,7 @@ __global__ void __launch_bounds__(kHalfThreads) k_half_area(HalfArgs a) {
             const bool inner = y > 0 && x > 0 && y < hm - 1 && x < wm - 1 && mask[k - wm] && mask[k + wm] &&
                                mask[k - 1] && mask[k + 1];
             if (!inner) {
-                ring[atomicAdd(&s_int[0], 1)] = cell[k];
+                if (!isnan(cell[k])) ring[atomicAdd(&s_int[0], 1)] = cell[k];
                 lmin = fmin(lmin, cell[k]);
             }
         }
@@ -2288,7 +2288,7 @@ __global__ void __launch_bounds__(kHalfThreads, 2) k_tail_area(TailArgs t) {
                 if (tid == 0) s_int[0] = 0;
                 __syncthreads();
                 for (int k = tid; k < area; k += kHalfThreads)
-                    if (mask[k] && lmask[k]) lv[atomicAdd(&s_int[0], 1)] = cell[k];
+                    if (mask[k] && lmask[k] && !isnan(cell[k])) lv[atomicAdd(&s_int[0], 1)] = cell[k];
                 __syncthreads();
                 const int r = s_int[0], k1 = (r - 1) / 2, k2 = r / 2;
                 for (int q0 = tid; q0 < r; q0 += kHalfThreads) {

@@ -178,3 +178,59 @@ def test_the_first_of_equal_peaks_is_taken(size):
     for out in (single, avg):
         np.testing.assert_allclose(out["center_local"].cpu().numpy(), want, atol=0.3)
     np.testing.assert_allclose(norm["centers"].cpu().numpy(), want, atol=0.3)
+
+
+@pytest.mark.parametrize("side", [9, 24, 33])
+def test_levels_leave_nan_pixels_out(side):
+    """NaN pixels (0 / 0 shares of the light where no model reaches) among the level pixels, all of them or some: the level
+    is the median of the others, NaN without any, and never another window's. Such a window has no signal. The level is
+    the middle value or the mean of two, as NumPy takes it: the same bits."""
+    import torch
+
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    rng = np.random.default_rng(side)
+    n = 592 * 2  # several windows a block, one after another
+    cells = rng.uniform(100, 900, (n, side, side)).astype(np.float32)
+    level = (rng.random((n, side, side)) < 0.4).astype(np.uint8)
+    ring = np.ones((side, side), bool)
+    ring[1:-1, 1:-1] = False
+    for i in range(n):
+        if i % 4 == 1:
+            cells[i][level[i] > 0] = np.nan
+            cells[i][ring] = np.nan
+        elif i % 4 == 3:
+            cells[i][rng.random((side, side)) < 0.5] = np.nan
+    ones = dev.upload(np.ones((n, side, side), np.uint8))
+    org = dev.upload(np.zeros((n, 2), np.int32))
+    win, level_d = dev.upload(cells), dev.upload(level)
+    vor = dev.upload(np.ascontiguousarray(np.repeat(np.arange(n, dtype=np.int32), side)[:, None] * np.ones((1, side), np.int32)))
+    boxes = dev.upload(np.column_stack((np.zeros(n), np.arange(n) * side, np.full(n, side), np.full(n, side))).astype(np.int32))
+    roi = dev.upload(cells.astype(np.float64))
+    op = _operator(side)
+    zy, zx_t = dev.upload(op), dev.upload(np.ascontiguousarray(op.T))
+    outs = [_outputs(n, 13) for _ in range(4)]
+    head = (win.data_ptr(), ones.data_ptr(), level_d.data_ptr(), ones.data_ptr(), org.data_ptr(), org.data_ptr(), n, side,
+            ANGLES)
+    none = (None,) * 4
+    ws = dev.workspace(max(_lib.size("spx_tail_area_workspace_bytes", side, 4, ANGLES),
+                           _lib.size("spx_half_area_workspace_bytes", side, side, 4)))
+    _lib.call("spx_tail_area_spline_cd", *head, 0.2, 16, 0, None, outs[0][1], *none, dev.stream_ptr())
+    _lib.call("spx_tail_area_cd", *head, zy.data_ptr(), zx_t.data_ptr(), 4, 0.2, 16, 0, None, outs[1][1], *none, ws.data_ptr(),
+              ws.numel(), dev.stream_ptr())
+    cell = (roi.data_ptr(), vor.data_ptr(), boxes.data_ptr(), None, n, side, side, side, ANGLES)
+    _lib.call("spx_half_area_spline_cd", *cell, 0.5, 1, 16, 0, outs[2][1], None, dev.stream_ptr())
+    _lib.call("spx_half_area_cd", *cell, zy.data_ptr(), zy.data_ptr(), 4, 0.5, 1, 16, 0, outs[3][1], None, ws.data_ptr(),
+              ws.numel(), dev.stream_ptr())
+    torch.cuda.synchronize()
+    import warnings
+
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore", RuntimeWarning)
+        values = cells.astype(np.float64).reshape(n, -1)
+        tail = np.nanmedian(np.where(level.reshape(n, -1) > 0, values, np.nan), axis=1)
+        half = np.nanmedian(np.where(ring.ravel()[None], values, np.nan), axis=1)
+    for (b, _), want in zip(outs, (tail, tail, half, half)):
+        np.testing.assert_array_equal(b["metrics"].cpu().numpy()[7], want)
+        assert (b["status"].cpu().numpy()[1::2] == b["status"].cpu().numpy()[1]).all()
