@@ -447,11 +447,10 @@ __global__ void __launch_bounds__(kFitWarpsMax * 32, 2) k_fit_initial(FitArgs a,
 // One deblending iteration for every cell: clean (image - background - (model - own)), LM from the
 // current params, relaxation p + relax * (fitted - p) (non-finite components step 0), status of
 // the relaxed params, and max |step[1:]| (NaN unless the cell is "ok" with a finite fit).
-// Px: the pixel type (a dtype branch per load cost 3 % of the kernel).
-// Bound: FP64 (54 % of its rate) and the latency behind it at 16 warps an SM. 96 registers in FP64 hold 20 warps
-// for 172 bytes of spills: 116k cells 4.45 -> 4.27 ms (80: 4.76; 9,800 cells of 30 px 151 -> 153 us).
-template <typename T, typename Px>
-__global__ void __maxnreg__(sizeof(T) == 8 ? 96 : 128) k_fit_iteration(FitArgs a, spx_bgmap bg, const double* model, int radius_cap,
+// Px: the pixel type (a dtype branch per load cost 3 % of the kernel). kRegs: registers a thread (fit_registers).
+// Bound: FP64 (54 % of its rate) and the latency behind it at 16 warps an SM.
+template <typename T, typename Px, int kRegs>
+__global__ void __maxnreg__(kRegs) k_fit_iteration(FitArgs a, spx_bgmap bg, const double* model, int radius_cap,
                                 const double* params, double relaxation, double* params_out,
                                 uint8_t* status_out, double* maxstep, int* iters) {
     extern __shared__ unsigned char smem[];
@@ -1284,15 +1283,32 @@ int launch_fit_initial(const FitArgs& a0, FitLayout L, cudaStream_t s, const dou
     }
 }
 
+// Registers of k_fit_iteration in FP64. At 96 (172 bytes of spills) an SM holds five blocks of four warps instead of
+// four, where their cells' shared memory allows: 116k cells of 24 px 4.45 -> 4.27 ms a launch, 7,200 274 -> 263 us (80:
+// 4.76 ms). That pays where the cells take fewer rounds of all warps for it: 2,800 cells of 24 px 133 -> 115 us (one round
+// for two), but 2,000 94 -> 113 us, 6,200 (three either way) 235 -> 240 us, and 3,100 cells of 36 px, three blocks of
+// whose data fill an SM, 240 -> 253 us.
+int fit_registers(int n, size_t smem, int warps) {
+    const int fit = smem ? (int)(228 * 1024 / (smem + kLmSlotBytes + 1024)) : 0;  // blocks an SM, by shared memory
+    auto rounds = [&](int regs) {
+        const int at_once = fit_sms() * warps * std::max(1, std::min(65536 / (regs * 32 * warps), fit));
+        return (n + at_once - 1) / at_once;
+    };
+    return rounds(96) < rounds(128) ? 96 : 128;
+}
+
 template <typename T, typename Px>
 int launch_fit_iteration_px(const FitArgs& a0, FitLayout L, cudaStream_t s, const spx_bgmap& bg, const double* model,
                             int radius_cap, const double* params, double relaxation, double* params_out,
                             uint8_t* status_out, double* maxstep, int* iterations) {
     return launch_fit(a0, L, s, [&](const FitArgs& fa, size_t smem, int warps, int blocks) -> int {
+        auto kernel = k_fit_iteration<T, Px, 128>;
+        if constexpr (sizeof(T) == 8)
+            if (fit_registers(fa.n, smem, warps) == 96) kernel = k_fit_iteration<T, Px, 96>;
         if (smem + kLmSlotBytes > 48 * 1024)
-            SPX_CUDA(cudaFuncSetAttribute(k_fit_iteration<T, Px>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_fit_iteration<T, Px><<<blocks, warps * 32, smem, s>>>(fa, bg, model, radius_cap, params, relaxation,
-                                                                 params_out, status_out, maxstep, iterations);
+            SPX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<blocks, warps * 32, smem, s>>>(fa, bg, model, radius_cap, params, relaxation, params_out, status_out, maxstep,
+                                                iterations);
         return check_launch("k_fit_iteration");
     });
 }
