@@ -970,12 +970,17 @@ k_refine(const void* img, int dtype, int H, int W, const int* labels, const int*
 // The log-quadratic refiner. A warp takes its blobs one after another as far as their sums, and solves up
 // to kLogquadBatch of them together, one per lane: the 6 x 6 elimination with its divisions is a serial chain
 // that all lanes of a warp would otherwise repeat for every single blob (more than half of the kernel).
-// Registers for six blocks an SM with integer images; the sort keys of the others leave room for four (with six the
-// 27 sums spill: 20,000 ROIs of 42 px of a float image 1158 us one blob after another, 1213 spilt, now 1048).
+// kBlocks an SM: six with integer images; four, so that the 27 sums stay in registers, where the rows fill no more
+// than four, and with other images, whose sort keys leave room for four (20,000 ROIs of 42 px of a float image 1158 us
+// one blob after another, 1213 with six, now 1048). Six and four blocks: one ROI of 136 px 421 and 341 us, 2,300 ROIs of
+// 18 px 24.0 and 19.5, 116,000 of 18 px 544 and 593. A table with a device count of its rows is counted as few up to the
+// 16,384 rows of a small frame, which seldom fills it.
+constexpr int kLogquadFew = 4 * 148 * kWarpsPerBlock;
+constexpr int kLogquadFewCounted = 16384;
 constexpr int kLogquadBatch = 16;
 
-template <typename Px>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, std::is_void<Px>::value ? 4 : 6)
+template <typename Px, int kBlocks>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kBlocks)
 k_refine_logquad(const void* img, int dtype, int H, int W, const int* labels, const int* rows, const uint8_t* methods,
                  int n, const int* n_dev, int fill, int pad, double* centers) {
     constexpr bool kInteger = !std::is_void<Px>::value;
@@ -1044,10 +1049,12 @@ int launch_refine(const void* img, int dtype, int H, int W, const int* labels, c
         constexpr int M = decltype(method)::value;
         if (err || !(which >> M & 1u)) return;
         using Px = std::remove_pointer_t<decltype(px)>;
-        if constexpr (M == SPX_REFINE_LOGQUAD)
-            k_refine_logquad<Px><<<blocks, kWarpsPerBlock * 32, 0, s>>>(img, dtype, H, W, labels, rows, methods, n, n_dev,
-                                                                        fill, pad, centers);
-        else
+        if constexpr (M == SPX_REFINE_LOGQUAD) {
+            auto kernel = k_refine_logquad<Px, 4>;
+            if constexpr (!std::is_void<Px>::value)
+                if (n > (n_dev ? kLogquadFewCounted : kLogquadFew)) kernel = k_refine_logquad<Px, 6>;
+            kernel<<<blocks, kWarpsPerBlock * 32, 0, s>>>(img, dtype, H, W, labels, rows, methods, n, n_dev, fill, pad, centers);
+        } else
             k_refine<M, Px><<<blocks, kWarpsPerBlock * 32, 0, s>>>(img, dtype, H, W, labels, rows, methods, n, n_dev, fill,
                                                                    pad, centers);
         fill = 0;

@@ -120,3 +120,27 @@ def test_large_rois_take_the_same_pixels_in_the_same_order(refine, w, h):
             y0, x0 = max(0, 2 - pad), max(0, 2 - pad)
             ys, xs = np.nonzero(m[y0:, x0:])
             np.testing.assert_array_equal(got[-1], [[x0 + xs.sum() / len(xs), y0 + ys.sum() / len(ys)]])
+
+
+@pytest.mark.parametrize("dtype", ["uint8", "uint16"])
+@pytest.mark.parametrize("pad", [0, 9])
+def test_logquad_does_not_depend_on_the_number_of_rows(dtype, pad):
+    """The same blobs as few rows, as many, and as tables with a device count on either side of 16,384 rows: the forms with
+    four and with six blocks per SM, staged regions and larger ones, bit for bit."""
+    from imageprocessor_new_b200 import _device as dev
+    from imageprocessor_new_b200 import _lib
+
+    img, labels, rows = _scene(dtype, 1)
+    k, code = len(rows), _lib.REFINE_CODES["logquad"]
+    img_d, lab_d = dev.upload(img), dev.upload(labels)
+    got = []
+    for times, counted in ((1, False), (30, False), (100, True), (140, True)):
+        n = k * times
+        rows_d, meth_d = dev.upload(np.tile(rows, (times, 1))), dev.upload(np.full(n, code, np.uint8))
+        out, live = dev.upload(np.full((n, 2), -7.0)), dev.upload(np.array([n], np.int32))
+        _lib.call("spx_refine_selected", img_d.data_ptr(), dev.dtype_code(img_d), *labels.shape, lab_d.data_ptr(),
+                  rows_d.data_ptr(), meth_d.data_ptr(), n, live.data_ptr() if counted else None, pad, code, out.data_ptr(),
+                  dev.stream_ptr())
+        got.append(out.cpu().numpy())
+        np.testing.assert_array_equal(got[-1], np.tile(got[0], (times, 1)))
+    assert np.isfinite(got[0]).all(axis=1).mean() > 0.3
