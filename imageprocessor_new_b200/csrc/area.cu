@@ -19,8 +19,8 @@
 // values, so each later step evaluates only the units that can hold what it looks for.
 //
 // Measured on one B200 against the dense kernels: the five tail methods of 4,032 windows of 59 px (both
-// passes) 80.3 -> 6.9 ms; half_area and half_area_min + _min_avg of the 7,225 cells of a 2047 x 2050 page
-// (24 px) 5.47 -> 1.42 ms.
+// passes) 80.3 -> 6.7 ms; half_area and half_area_min + _min_avg of the 7,225 cells of a 2047 x 2050 page
+// (24 px) 5.47 -> 1.41 ms.
 
 #include <algorithm>
 
@@ -213,7 +213,7 @@ __device__ __forceinline__ float key_float(unsigned k) {
 // thread, and the units' upper bounds. top->x: the first sub-pixel in row-major order that reaches it to rounding (a
 // margin of 2^-48, twice the sums' error): equal peaks of a cell (isolated pixels of one value, mirrored holes) differ
 // in the last bits of the recursion's sums, and the reference takes the first of equal ones. It is looked up over the
-// few units that reach the peak (2-3 % of the kernels).
+// few units that reach the peak, each found by a lane (half_area 1.38 -> 1.41 ms, tail windows as before).
 template <int NT>
 __device__ void area_peak(const AreaCta<NT>& h, double* s_red, int* s_ired, double* top_v, int2* top) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = h.g.RW;
@@ -262,18 +262,21 @@ __device__ void area_peak(const AreaCta<NT>& h, double* s_red, int* s_ired, doub
     __syncthreads();
     const double reach = best - 0x1p-48 * best;
     int first = best_i;
+    const int units = h.g.hm * RW;
     if (best > 0.0 && isfinite(best))
-        for (int ky = warp; ky < h.g.hm; ky += NT / 32)
-            for (int w = 0; w < RW; ++w) {
-                if ((double)h.unit[ky * RW + w] < reach) continue;
+        for (int u0 = warp * 32; u0 < units; u0 += NT) {
+            const bool reaches = u0 + lane < units && (double)h.unit[min(u0 + lane, units - 1)] >= reach;
+            for (unsigned b = __ballot_sync(0xffffffffu, reaches); b; b &= b - 1) {
+                const int u = u0 + __ffs(b) - 1, ky = u / RW, w = u - ky * RW;
                 const int X = min(w * 32 + lane, h.g.Wb - 1);
                 double v[4];
                 unit_values(h.coef, h.g.cp, ky, X, v);
-                if (!((h.pmask[ky * RW + w] >> lane) & 1u)) continue;
+                const bool in = (h.pmask[u] >> lane) & 1u;
 #pragma unroll
                 for (int p = 0; p < 4; ++p)
-                    if (v[p] >= reach) first = min(first, (kF * ky + p) * h.g.Wb + X);
+                    if (in && v[p] >= reach) first = min(first, (kF * ky + p) * h.g.Wb + X);
             }
+        }
     first = __reduce_min_sync(0xffffffffu, first);
     if (lane == 0) s_ired[warp] = first;
     __syncthreads();
